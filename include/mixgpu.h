@@ -355,7 +355,8 @@ int mgpu_cg_jacobi_noalloc(int n, const int32_t* d_row_ptr, const int32_t* d_col
                            int* it, double* res, int* ierr);
 
 /* Launch tunables, process-wide (for autotuning): "single_block_rows" (a
- * solve of at most this many rows runs in one block, default 32768),
+ * solve of at most this many rows runs in one block, default 32768; mixed
+ * systems that fit in the SMs' shared memory are divided by their size alone),
  * "sweep_threads" (threads of a sync-free triangular sweep, default 65536),
  * "sweep_sleep_ns" (back-off of a long wait in that sweep, default 0),
  * "min_blocks" (least number of blocks of a multi-block solve, default 1),
@@ -371,7 +372,8 @@ int mgpu_cg_jacobi_noalloc(int n, const int32_t* d_row_ptr, const int32_t* d_col
  * now: creating one later waits for kernels on other streams),
  * "l2_prefetch_mb" (mixed form: a system, or the systems of a batched phase
  * together, streaming more than this many MB per SpMV pass prefetch each
- * tile's successor into L2, default 96), "mixed_blocks_per_sm" (mixed and FP64
+ * tile's successor into L2, default 96), "mixed_blocks_per_sm" (mixed, when the
+ * system does not fit in the SMs' shared memory, and FP64
  * polynomial single-system solves: 2-8 resident blocks of 256 threads per SM
  * (the FP64 polynomial form 2-5), the register budget sized to match,
  * default 5), "batch_blocks_per_sm" (the

@@ -17,10 +17,10 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libmixgpu.so")
 BUILD = os.path.join(HERE, "_build")
 
-SOURCES = ["case.cu", "assembly.cu", "krylov.cu", "krylov_mixed.cu", "krylov_poly64.cu", "batch.cu", "standalone.cu", "noalloc.cu", "device_topo.cu",
+SOURCES = ["case.cu", "assembly.cu", "krylov.cu", "krylov_mixed.cu", "krylov_resident.cu", "krylov_poly64.cu", "batch.cu", "standalone.cu", "noalloc.cu", "device_topo.cu",
            "mesh_host.cpp", "cas_reader.cpp"]
 # the mixed-precision form needs no bit-parity and may contract into FMA
-FMA_OK = {"krylov_mixed.cu", "krylov_poly64.cu"}
+FMA_OK = {"krylov_mixed.cu", "krylov_resident.cu", "krylov_poly64.cu"}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-ffp-contract=off", "--expt-relaxed-constexpr"]

@@ -247,7 +247,7 @@ MixedArgs mixed_args(const MgpuCase* c, bool bicg) {
   return MixedArgs{c->d.a32,   c->d.dinv32, c->d.w32,  c->ctrl.mixed_tol > 0.0 ? c->ctrl.mixed_tol : 1e-4,
                    k,          ratio,       c->d.ell_w, c->d.ell_col, c->d.ell_val,
                    c->d.red32, (c->d.ell_col && big) ? 1 : 0, 0.0, c->d.ell_ld, 0,
-                   c->d.ell_val64};
+                   c->d.ell_val64, c->d.plan};
 }
 
 // The same solves in FP64 throughout (MGPU_PREC_FP64_POLY): PCG keeps one
@@ -686,9 +686,9 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
   if ((e = ensure_recs(c, 64))) return fail(e);
   if (poly) {
     // column-major ELL copy of the pattern for the polynomial forms' SpMV (rows of at most 8 entries)
-    int w = 0, *ell = nullptr;
+    int w = 0, bw = 0, *ell = nullptr;
     long ld = 0;
-    if ((e = device_ell(d.N, d.row_ptr, d.col, 8, w, ld, ell, keep, c->stream))) return fail(e);
+    if ((e = device_ell(d.N, d.row_ptr, d.col, 8, w, ld, ell, keep, c->stream, &bw))) return fail(e);
     if (ell) {
       d.ell_col = ell;
       // values zero in the padding rows
@@ -699,6 +699,7 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
       if (ctrl->precision == MGPU_PREC_MIXED) {
         if ((e = c->alloc(d.ell_val, (size_t)w * ld))) return fail(e);
         MGPU_CUDA(cudaMemsetAsync(d.ell_val, 0, sizeof(float) * (size_t)w * ld, c->stream));
+        if ((e = plan_resident(d.N, w, (int)ld, ell, bw, d.plan, c->stream))) return fail(e);
       }
       d.ell_w = w;
       d.ell_ld = (int)ld;

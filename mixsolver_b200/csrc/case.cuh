@@ -68,6 +68,13 @@ struct KrylovArgs {
   int sweep_sleep;     // nanosleep of a long wait in that sweep (0: spin)
 };
 
+// How a system is divided for its resident solves (krylov_resident.cu): rows of
+// a block (0: the system does not fit), most 32-row words a block reads of
+// other blocks, largest |column - row|.
+struct ResidentPlan {
+  int rows = 0, words = 0, bw = 0;
+};
+
 // Data of a polynomial-preconditioned solve in working precision V: the
 // matrix copy and inverse diagonal in V, work vectors in V (10 N), inner
 // relative tolerance. V = float is the mixed-precision form (FP32 inner
@@ -93,6 +100,7 @@ struct MixedArgsT {
   // the mixed form's PCG (V = float): the FP64 values in the ELL layout, for
   // the FP64 conjugate-gradient product q = A p (null: the CSR values)
   double* ell64;
+  ResidentPlan plan;  // krylov_resident.cu (rows 0: no resident solve)
 };
 using MixedArgs = MixedArgsT<float>;
 
@@ -193,6 +201,7 @@ struct DeviceCase {
   double *a64 = nullptr, *dinv64 = nullptr, *w64 = nullptr, *ell_val64 = nullptr;  // FP64 polynomial form
   int ell_w = 0;
   int ell_ld = 0;  // ELL leading dimension: N rounded up to a multiple of 4
+  ResidentPlan plan;
   double* red32 = nullptr;  // chunk reduction partials of the mixed-precision solves
   // Krylov work
   double *kw = nullptr;  // 10*N
@@ -220,6 +229,9 @@ int launch_krylov_pcg(const KrylovArgs& a, cudaStream_t s);
 int launch_factor(const KrylovArgs& a, int kind, cudaStream_t s);
 int krylov_grid(int n, int& block, int which);
 int launch_pcg_mixed(const KrylovArgs& a, const MixedArgs& m, cudaStream_t s);
+// pattern symmetric, ell_col of W entries a row; waits for stream s
+int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan& plan, cudaStream_t s);
+int launch_resident(const KrylovArgs& a, const MixedArgs& m, bool pcg, cudaStream_t s, bool* taken);
 int launch_bicgstab_mixed(const KrylovArgs& a, const MixedArgs& m, cudaStream_t s);
 int launch_pcg_poly64(const KrylovArgs& a, const MixedArgsT<double>& m, cudaStream_t s);
 int launch_bicgstab_poly64(const KrylovArgs& a, const MixedArgsT<double>& m, cudaStream_t s);

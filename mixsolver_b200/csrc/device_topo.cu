@@ -363,9 +363,21 @@ __global__ void k_reverse(int N, const int* __restrict__ order, int* new_of_old)
 
 // ---------------- per-case lists ------------------------------------------
 
-__global__ void k_row_width(int N, const int* __restrict__ rp, int* w) {
+// w[0]: the widest row; w[1]: the largest |column - row|
+__global__ void k_row_width(int N, const int* __restrict__ rp, const int* __restrict__ col, int* w) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) atomicMax(w, rp[i + 1] - rp[i]);
+  int wide = 0, far = 0;
+  if (i < N) {
+    const int b = rp[i], e = rp[i + 1];
+    wide = e - b;
+    for (int k = b; k < e; ++k) far = max(far, abs(col[k] - i));
+  }
+  wide = __reduce_max_sync(0xffffffffu, wide);
+  far = __reduce_max_sync(0xffffffffu, far);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(w, wide);
+    atomicMax(w + 1, far);
+  }
 }
 
 // column-major ELL pattern: entry t of row i at t * ld + i, padding the row
@@ -492,14 +504,18 @@ int device_topology(int N, int F, const int* c0, const int* c1, DeviceTopo& t, c
 }
 
 int device_ell(int N, const int* rp, const int* col, int max_width, int& W, long& ld, int*& ell,
-               const TopoAlloc& alloc, cudaStream_t s) {
+               const TopoAlloc& alloc, cudaStream_t s, int* bandwidth) {
   Tmp T(s);
   int* w = nullptr;
-  DT_TRY(T.get(w, 1));
-  MGPU_CUDA(cudaMemsetAsync(w, 0, sizeof(int), s));
-  k_row_width<<<ceil_div(N, 256), 256, 0, s>>>(N, rp, w);
+  DT_TRY(T.get(w, 2));
+  MGPU_CUDA(cudaMemsetAsync(w, 0, 2 * sizeof(int), s));
+  k_row_width<<<ceil_div(N, 256), 256, 0, s>>>(N, rp, col, w);
   MGPU_LAUNCH_CHECK("k_row_width");
-  DT_TRY(read_int(w, W, s));
+  int h[2] = {0, 0};
+  MGPU_CUDA(cudaMemcpyAsync(h, w, sizeof(h), cudaMemcpyDeviceToHost, s));
+  MGPU_CUDA(cudaStreamSynchronize(s));
+  W = h[0];
+  if (bandwidth) *bandwidth = h[1];
   ell = nullptr;
   ld = ((long)N + 3) / 4 * 4;  // each column starts on a 16-byte boundary
   if (W > max_width) return 0;

@@ -31,8 +31,9 @@ int device_topology(int N, int F, const int* c0, const int* c1, DeviceTopo& t, c
 // Widest row W of the pattern and, when W <= max_width, its column-major ELL
 // copy: entry t of row i at t * ld + i with ld = N rounded up to a multiple of
 // 4 (every column starts 16-byte aligned), padding the row itself.
+// *bandwidth (optional): the pattern's largest |column - row|.
 int device_ell(int N, const int* row_ptr, const int* col, int max_width, int& W, long& ld, int*& ell,
-               const TopoAlloc& alloc, cudaStream_t s);
+               const TopoAlloc& alloc, cudaStream_t s, int* bandwidth = nullptr);
 // Each cell's boundary faces that carry a group, in the order of its face list.
 int device_boundary_lists(int N, const int* cf_ptr, const int* cf, const int* c1, const int* fgrp, int*& bf_ptr,
                           int*& bf, const TopoAlloc& alloc, cudaStream_t s);

@@ -143,6 +143,9 @@ const void* batch_kernel(bool pcg, int ell, int occ) {
 }  // namespace
 
 int launch_pcg_mixed(const KrylovArgs& a, const MixedArgs& m, cudaStream_t s) {
+  bool taken = false;  // systems that fit in the SMs' shared memory: krylov_resident.cu
+  if (int e = launch_resident(a, m, true, s, &taken)) return e;
+  if (taken) return 0;
   const int ell = ell_mode(m);
   const void* one = ell == 0 ? (const void*)k_pcg_mixed<true, 0> : (const void*)k_pcg_mixed<true, 1>;
   const void* grid = by_occ8(g_mixed_occ, [&](auto o) {
@@ -154,6 +157,9 @@ int launch_pcg_mixed(const KrylovArgs& a, const MixedArgs& m, cudaStream_t s) {
 }
 
 int launch_bicgstab_mixed(const KrylovArgs& a, const MixedArgs& m, cudaStream_t s) {
+  bool taken = false;
+  if (int e = launch_resident(a, m, false, s, &taken)) return e;
+  if (taken) return 0;
   const int ell = ell_mode(m);
   const void* one = ell == 0 ? (const void*)k_bicgstab_mixed<true, 0> : (const void*)k_bicgstab_mixed<true, 1>;
   const void* grid = by_occ8(g_mixed_occ, [&](auto o) {

@@ -1,0 +1,869 @@
+// krylov_resident.cu -- the mixed form's solves for systems that fit in the
+// SMs' shared memory: the pressure PCG (FP64 conjugate gradients with the FP32
+// Chebyshev-Jacobi polynomial) and the momentum BiCGStab of krylov_poly.cuh,
+// bit for bit the same numbers, with another division of the work.
+//
+// What bounds the streaming kernels (k_pcg_mixed) on such systems is neither
+// HBM nor arithmetic: a Chebyshev pass of a few hundred thousand rows costs a
+// grid barrier (every block's stores made visible, one counter, polls) plus
+// two dependent trips to L2 per row, whatever the row count. Here
+//   - a block owns a contiguous range of rows (whole super-chunks) for the
+//     whole solve and keeps its rows of the FP32 matrix and 16-bit local
+//     column numbers in shared memory and its part of the polynomial's vectors
+//     in registers;
+//   - between two passes only the values other blocks need move: each row's
+//     new value goes to global memory in one 8-byte word together with the
+//     number of its exchange, and a block reads the words its rows refer to
+//     until they carry that number. The data is its own signal, so a pass has
+//     no barrier and no fence (the words are written and read by relaxed
+//     64-bit accesses, which are single-copy atomic). Only the sums
+//     take a barrier (exchanged as words too, they were slower from about a
+//     hundred blocks on, each polling every block's sums);
+//   - the words a block needs are found in the prologue: the 32-row words its
+//     columns touch, in the window [first row - bw, last row + bw], bw = the
+//     largest |column - row|.
+// The sums keep the layout-independent tree of krylov_poly.cuh.
+//
+// Measured on a B200, one PCG iteration at degree 24 (streaming kernel ->
+// here): 6,400 rows 243 -> 32 us, 42,253 rows 99 -> 42 us, 82,944 rows (5
+// entries) 93 -> 42 us, 524,288 rows 181 -> 116 us; a BiCGStab iteration 42,253
+// rows 24 -> 11 us, 524,288 rows 46 -> 33 us. A pass of the 524,288 rows is
+// 1.7 us of shared-memory reads (48 B of matrix and 7 gathers a row) and 1.9 us
+// of exchange. One block of 512 threads per SM: two blocks of 512 (64
+// registers each, one computing while the other's words travel) and one of
+// 1024 were 10-25 % slower, by their spills.
+
+#include <algorithm>
+
+#include "exchange.cuh"
+#include "krylov_poly.cuh"
+
+namespace mgpu {
+namespace {
+
+constexpr int kResidentThreads = 512;  // of a block, at most: 128 registers each
+constexpr int kHaloRegs = 4;   // halo words of a warp whose rows stay in registers
+constexpr int kHaloBatch = 16; // halo words of a warp whose polls are in flight together, at most
+
+// What a block keeps for the whole solve: its rows in shared memory (byte
+// offsets into it) and the words it exchanges. The window starts at offset 0:
+// R own values, then 32 per halo word.
+template <int WC>
+struct Resident {
+  int n, R, start, end;  // rows of the system, of a block, this block's range
+  int wb, nhw, nb;       // first row of the window, halo words, blocks
+  int cp, cps;           // chunk sums (2 x cps doubles)
+  int va;                // float4: entries 0..3
+  int vb;                // 7: float4, entries 4..6 and the inverse diagonal; 5: float2, entry 4 and the inverse diagonal
+  int ia;                // 7: uint4, window byte offsets of columns 0..6, 16 bits each; 5: uint2, of columns 0..3
+  int ib;                // 5: unsigned short, of column 4
+  int words;             // unsigned short: halo word k covers rows wb + 32 * word ...
+  int nsc;
+  unsigned seq, rseq;    // exchanges and sums so far
+  u64* ll;               // exchange words (2 parities of n)
+  double* sums;          // super-chunk sums (2 halves x 2 sums x nsc)
+  int hpw;               // halo words per warp, rounded up
+  int hrow[kHaloRegs];   // the rows this lane polls for the warp's first halo words
+};
+
+// Shared memory of a block (bytes); nhw halo words, window of wwin words.
+__host__ __device__ inline int resident_win_bytes(int R, int nhw, int wwin) {
+  const int win = 4 * R + 128 * (nhw + 1), scratch = 4 * wwin;  // the prologue's word ranks, in the window's place
+  return ((win > scratch ? win : scratch) + 15) & ~15;
+}
+__host__ __device__ inline int resident_window_words(int R, int bw) { return R / 32 + 2 * ((bw + 31) / 32); }
+__host__ __device__ inline int resident_smem(int WC, int R, int bw, int nhw, int cps) {
+  return resident_win_bytes(R, nhw, resident_window_words(R, bw)) + 16 * cps + (WC == 7 ? 48 : 34) * R + 2 * nhw;
+}
+
+template <int WC>
+__device__ __forceinline__ void resident_views(Resident<WC>& m, int R, int bw, int nhw, int cps) {
+  m.cp = resident_win_bytes(R, nhw, resident_window_words(R, bw));
+  m.cps = cps;
+  m.va = m.cp + 16 * cps;
+  m.vb = m.va + 16 * R;
+  m.ia = m.vb + (WC == 7 ? 16 : 8) * R;
+  m.ib = m.ia + (WC == 7 ? 16 : 8) * R;
+  m.words = m.ib + (WC == 7 ? 0 : 2) * R;
+}
+
+__device__ __forceinline__ float win_at(unsigned off) {
+  return *reinterpret_cast<const float*>(block_smem + off);
+}
+
+// f(entry, byte offset of its column in the window) over the row's entries
+template <int WC, typename F>
+__device__ __forceinline__ void resident_cols(const Resident<WC>& m, int l, F&& f) {
+  if constexpr (WC == 7) {
+    const uint4 c = smem_at<uint4>(m.ia, l);
+    f(0, c.x & 0xffffu);
+    f(1, c.x >> 16);
+    f(2, c.y & 0xffffu);
+    f(3, c.y >> 16);
+    f(4, c.z & 0xffffu);
+    f(5, c.z >> 16);
+    f(6, c.w);
+  } else {
+    const uint2 c = smem_at<uint2>(m.ia, l);
+    f(0, c.x & 0xffffu);
+    f(1, c.x >> 16);
+    f(2, c.y & 0xffffu);
+    f(3, c.y >> 16);
+    f(4, (unsigned)smem_at<unsigned short>(m.ib, l));
+  }
+}
+
+// One row of the FP32 product: entries in ELL order as in spmv32_rows (entries
+// past the row's width are value 0 at the row itself).
+template <int WC>
+__device__ __forceinline__ float resident_row(const Resident<WC>& m, int l, float& dinv) {
+  float v[WC];
+  const float4 a = smem_at<float4>(m.va, l);
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = a.z;
+  v[3] = a.w;
+  if constexpr (WC == 7) {
+    const float4 b = smem_at<float4>(m.vb, l);
+    v[4] = b.x;
+    v[5] = b.y;
+    v[6] = b.z;
+    dinv = b.w;
+  } else {
+    const float2 b = smem_at<float2>(m.vb, l);
+    v[4] = b.x;
+    dinv = b.y;
+  }
+  float acc = 0.0f;
+  resident_cols<WC>(m, l, [&](int t, unsigned off) { acc = fmaf(v[t], win_at(off), acc); });
+  return acc;
+}
+
+// The row's inverse diagonal.
+template <int WC>
+__device__ __forceinline__ float resident_dinv(const Resident<WC>& m, int l) {
+  if constexpr (WC == 7)
+    return smem_at<float4>(m.vb, l).w;
+  else
+    return smem_at<float2>(m.vb, l).y;
+}
+
+// The rows row[0 .. HB) of this lane, polled until they carry number seq, into
+// the window from halo word w0 in steps of the block's warps. Straight-line: a
+// taken branch a word costs more than the word (nhw = 6 words with 16 guarded
+// polls: 1.09 us an exchange, with 8: 0.74 us); words and lanes past the halo
+// poll a row of this block instead and land in the window's spare word.
+template <int HB, int WC>
+__device__ __forceinline__ bool halo_fetch(const Resident<WC>& S, const u64* llb, unsigned seq,
+                                           const int* row, int w0, DevStatus* st) {
+  const int T = blockDim.x, lane = threadIdx.x & 31, nw = T >> 5;
+  u64 v[HB];
+#pragma unroll
+  for (int q = 0; q < HB; ++q) v[q] = ld_word(llb + row[q]);
+  unsigned spins = 0;
+  while (true) {
+    unsigned bad = 0u;
+#pragma unroll
+    for (int q = 0; q < HB; ++q) bad |= (unsigned)(v[q] >> 32) ^ seq;
+    if (bad == 0u) break;
+    if (!keep_polling(spins, st)) return false;
+#pragma unroll
+    for (int q = 0; q < HB; ++q)
+      if ((unsigned)(v[q] >> 32) != seq) v[q] = ld_word(llb + row[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < HB; ++q)
+    smem_at<float>(0, S.R + 32 * min(w0 + q * nw, S.nhw) + lane) = __uint_as_float((unsigned)v[q]);
+  return true;
+}
+
+// The row lane polls for halo word w.
+template <int WC>
+__device__ __forceinline__ int halo_row(const Resident<WC>& S, int w) {
+  const int lane = threadIdx.x & 31;
+  const int own = min(S.start + lane, S.end - 1);
+  const int row = w < S.nhw ? S.wb + 32 * (int)smem_at<unsigned short>(S.words, w) + lane : own;
+  return row < S.n ? row : own;
+}
+
+// One exchange: this block's new values z (registers) go to its exchange words
+// and its own window, the halo words are read until they carry this exchange's
+// number; between() runs while they travel. Words of the other parity may
+// still be read by a slower neighbour; these are free: a block writes exchange
+// s + 2 only after it has read the words s + 1 of every block it exchanges
+// with (the pattern is symmetric), which those wrote after reading all of
+// their words s. Returns false when a bounded poll ran out.
+template <int WC, int K, typename F>
+__device__ __forceinline__ bool resident_exchange(Resident<WC>& S, const float (&z)[K], DevStatus* st, F&& between) {
+  const int T = blockDim.x, tid = threadIdx.x, warp = tid >> 5, nw = T >> 5;
+  const unsigned seq = ++S.seq;
+  u64* llb = S.ll + (long)(seq & 1u) * S.n;
+  if (S.nb > 1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = S.start + k * T + tid;
+      if (i < S.end) st_word(llb + i, pack_word(__float_as_uint(z[k]), seq));
+    }
+  }
+  between();
+  __syncthreads();  // the pass's reads of the window are done
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int l = k * T + tid;
+    if (l < S.R) smem_at<float>(0, l) = z[k];
+  }
+  // the polls start only now: sent right after the stores, the first ones come
+  // back before the neighbours' words
+  bool ok = true;
+  if (S.hpw > 0) {
+    if (S.hpw <= 1)
+      ok = halo_fetch<1>(S, llb, seq, S.hrow, warp, st);
+    else if (S.hpw <= 2)
+      ok = halo_fetch<2>(S, llb, seq, S.hrow, warp, st);
+    else if (S.hpw <= 4)
+      ok = halo_fetch<4>(S, llb, seq, S.hrow, warp, st);
+    else
+      for (int w0 = warp; w0 < S.nhw && ok; w0 += kHaloBatch * nw) {
+        int row[kHaloBatch];
+        if (w0 + 8 * nw >= S.nhw) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) row[q] = halo_row(S, w0 + q * nw);
+          ok = halo_fetch<8>(S, llb, seq, row, w0, st);
+        } else {
+#pragma unroll
+          for (int q = 0; q < kHaloBatch; ++q) row[q] = halo_row(S, w0 + q * nw);
+          ok = halo_fetch<kHaloBatch>(S, llb, seq, row, w0, st);
+        }
+      }
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
+// The block's rows into shared memory: the window's halo words, ranked in
+// ascending order, the window offsets of the columns, the FP32 values and
+// inverse diagonals; the FP64 ELL values (PCG); the exchange words cleared
+// (the barrier puts every block's clears before the first exchange); b.b and
+// the count of zero diagonals.
+template <int WC, int K, bool PCG>
+__device__ __forceinline__ bool resident_prologue(const KrylovArgs& a, const MixedArgs& m, VGrid& g, Resident<WC>& S, double& bnrm,
+                                  bool& diag_bad) {
+  const int T = blockDim.x, tid = threadIdx.x, s0 = S.start, e0 = s0 + S.R;
+  const int lane = tid & 31, warp = tid >> 5, nw = T >> 5;
+  const int W = m.ell_w, ld = m.ell_ld;
+  S.wb = max(0, s0 - (m.plan.bw + 31) / 32 * 32);
+  const int nwords = (min(S.n, e0 + m.plan.bw) - S.wb + 31) / 32;
+  unsigned* rank_of = reinterpret_cast<unsigned*>(block_smem);
+  __shared__ unsigned s_warp[32];
+  __shared__ unsigned s_run;
+  for (int w = tid; w < nwords; w += T) rank_of[w] = 0u;
+  if (tid == 0) s_run = 0u;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = s0 + k * T + tid;
+    if (i < S.end)
+#pragma unroll
+      for (int t = 0; t < WC; ++t)
+        if (t < W) {
+          const int c = m.ell_col[t * ld + i];
+          if (c < s0 || c >= e0) rank_of[(c - S.wb) >> 5] = 1u;  // every writer stores the same value
+        }
+  }
+  __syncthreads();
+  for (int w0 = 0; w0 < nwords; w0 += T) {
+    const int w = w0 + tid;
+    const bool on = w < nwords && rank_of[w] != 0u;
+    const unsigned bal = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) s_warp[warp] = __popc(bal);
+    __syncthreads();
+    unsigned before = s_run;
+    for (int q = 0; q < warp; ++q) before += s_warp[q];
+    const unsigned rank = before + __popc(bal & ((1u << lane) - 1u));
+    __syncthreads();
+    if (tid == T - 1) s_run = before + __popc(bal);
+    if (on) {
+      rank_of[w] = rank;
+      smem_at<unsigned short>(S.words, (int)rank) = (unsigned short)w;
+    }
+    __syncthreads();
+  }
+  S.nhw = (int)s_run;
+  S.hpw = (S.nhw + nw - 1) / nw;
+#pragma unroll
+  for (int q = 0; q < kHaloRegs; ++q) S.hrow[q] = halo_row(S, warp + q * nw);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int l = k * T + tid, i = s0 + l;
+    double c[2] = {0.0, 0.0};
+    float v[WC];
+    unsigned lc[WC];
+    float dv = 0.0f;
+#pragma unroll
+    for (int t = 0; t < WC; ++t) {
+      v[t] = 0.0f;
+      lc[t] = 4u * (unsigned)l;
+    }
+    if (i < S.end) {
+      const int rb = a.row_ptr[i], nr = a.row_ptr[i + 1] - rb;
+#pragma unroll
+      for (int t = 0; t < WC; ++t)
+        if (t < W) {
+          const double av = t < nr ? a.aval[rb + t] : 0.0;
+          v[t] = (float)av;
+          if (PCG) m.ell64[t * ld + i] = av;  // q = A p
+          const int cc = m.ell_col[t * ld + i];
+          lc[t] = 4u * (cc >= s0 && cc < e0
+                            ? (unsigned)(cc - s0)
+                            : (unsigned)S.R + 32u * rank_of[(cc - S.wb) >> 5] + (unsigned)((cc - S.wb) & 31));
+        }
+      if (a.zero_x) a.x[i] = 0.0;
+      const double dg = a.aval[a.diag[i]];
+      if (fabs(dg) < DTINY) c[1] = 1.0;
+      dv = (float)(1.0 / dg);
+      c[0] = a.b[i] * a.b[i];
+      S.ll[i] = 0ull;
+      S.ll[(long)S.n + i] = 0ull;
+    }
+    if (l < S.R) {
+      smem_at<float4>(S.va, l) = make_float4(v[0], v[1], v[2], v[3]);
+      if constexpr (WC == 7) {
+        smem_at<float4>(S.vb, l) = make_float4(v[4], v[5], v[6], dv);
+        smem_at<uint4>(S.ia, l) = make_uint4(lc[0] | lc[1] << 16, lc[2] | lc[3] << 16, lc[4] | lc[5] << 16, lc[6]);
+      } else {
+        smem_at<float2>(S.vb, l) = make_float2(v[4], dv);
+        smem_at<uint2>(S.ia, l) = make_uint2(lc[0] | lc[1] << 16, lc[2] | lc[3] << 16);
+        smem_at<unsigned short>(S.ib, l) = (unsigned short)lc[4];
+      }
+    }
+    resident_put<2>(S.cp, S.cps, k, c);
+  }
+  if (!vg_sync(g, a.st)) return false;
+  double v[2];
+  if (!resident_total<2>(S, g, a.st, v)) return false;
+  bnrm = sqrt(v[0]);
+  diag_bad = v[1] != 0.0;
+  return true;
+}
+
+__shared__ float2 s_cheb[64];  // the polynomial's recurrence coefficients
+
+// The Chebyshev-Jacobi polynomial of cheb_apply on the block's rows: on entry
+// z holds z0 (registers, exchanged); on return z is the result, exchanged, and
+// rz the sum r64.z.
+template <int WC, int K>
+__device__ __forceinline__ bool resident_cheb(Resident<WC>& S, VGrid& g, DevStatus* st, int degree, const float (&rr)[K],
+                                              float (&z)[K], const double* r64, double& rz) {
+  const int T = blockDim.x, tid = threadIdx.x;
+  float d[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) d[k] = z[k];
+  for (int j = 1; j < degree; ++j) {
+    const float2 c = s_cheb[j];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int l = k * T + tid;
+      if (l < S.R) {
+        float dinv;
+        const float az = resident_row<WC>(S, l, dinv);
+        const float res = dinv * (rr[k] - az);
+        d[k] = fmaf(c.x, d[k], c.y * res);
+        z[k] = z[k] + d[k];
+      }
+    }
+    if (j == degree - 1) break;
+    if (!resident_exchange<WC, K>(S, z, st, [] {})) return false;
+  }
+  // the result and its sum travel together
+  if (!resident_exchange<WC, K>(S, z, st, [&] {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const int i = S.start + k * T + tid;
+          const double c[1] = {i < S.end ? r64[i] * (double)z[k] : 0.0};
+          resident_put<1>(S.cp, S.cps, k, c);
+        }
+        total_post<1>(S, g);
+      }))
+    return false;
+  double t[1];
+  if (!total_wait<1>(S, g, st, t)) return false;
+  rz = t[0];
+  return true;
+}
+
+// pcg_hybrid (krylov_poly.cuh) on resident rows: the same recurrences, sums
+// and decisions.
+template <int WC, int K>
+__device__ __forceinline__ void resident_pcg(const KrylovArgs& a, const MixedArgs& m, VGrid& g, Resident<WC>& S, double bnrm,
+                             double rnorm0, float inv_th) {
+  const int T = blockDim.x, tid = threadIdx.x, ld = m.ell_ld, W = m.ell_w;
+  double *rs = a.r, *p = a.p, *pn = a.s;  // the direction is double-buffered
+  const double* __restrict__ ev = m.ell64;
+  const double sc = 1.0 / rnorm0;
+  const double stop = a.tol * bnrm * sc;
+  const double stop2 = stop * stop;
+  float z[K], rr[K];
+  double pk[K], qk[K];
+  // row i of the scaled residual: its FP32 copy and the first Chebyshev term
+  auto begin_row = [&](int k, int i, double ri) {
+    rs[i] = ri;
+    rr[k] = (float)ri;
+    z[k] = resident_dinv<WC>(S, k * T + tid) * rr[k] * inv_th;
+  };
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = S.start + k * T + tid;
+    z[k] = rr[k] = 0.0f;
+    if (i < S.end) begin_row(k, i, ldv(&a.r[i]) * sc);
+  }
+  if (!resident_exchange<WC, K>(S, z, a.st, [] {})) return;
+  double rz = 0.0, rnorm = rnorm0;
+  int total = 0, ierr = 0;
+  bool first = true;
+  while (true) {
+    double rzn;
+    if (!resident_cheb<WC, K>(S, g, a.st, m.cheb_k, rr, z, rs, rzn)) return;
+    double beta = 0.0;
+    if (!first) {
+      if (fabs(rz) < DTINY) {
+        ierr = 2;
+        break;
+      }
+      beta = rzn / rz;
+    }
+    rz = rzn;
+    ++total;
+    // pn := z + beta p, q := A pn: z from the window, p of the rows' columns
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int l = k * T + tid, i = S.start + l;
+      double c[1] = {0.0};
+      pk[k] = qk[k] = 0.0;
+      if (i < S.end) {
+        double v[WC], x[WC];
+        resident_cols<WC>(S, l, [&](int t, unsigned off) {
+          v[t] = t < W ? ev[t * ld + i] : 0.0;
+          const int lc = (int)(off >> 2);
+          const int col = lc < S.R ? S.start + lc : S.wb + 32 * (int)smem_at<unsigned short>(S.words, (lc - S.R) >> 5) + (lc & 31);
+          x[t] = first ? 0.0 : ldv(&p[col]);
+        });
+        resident_cols<WC>(S, l, [&](int t, unsigned off) {
+          const double zt = (double)win_at(off);
+          x[t] = first ? zt : fma(beta, x[t], zt);
+        });
+        double acc = 0.0;
+#pragma unroll
+        for (int t = 0; t < WC; ++t)
+          if (t < W) acc = fma(v[t], x[t], acc);
+        const double pi = first ? (double)z[k] : fma(beta, p[i], (double)z[k]);
+        pn[i] = pi;
+        pk[k] = pi;
+        qk[k] = acc;
+        c[0] = pi * acc;
+      }
+      resident_put<1>(S.cp, S.cps, k, c);
+    }
+    {
+      double* t = p;
+      p = pn;
+      pn = t;
+    }
+    first = false;
+    double pq[1];
+    if (!resident_total<1>(S, g, a.st, pq)) return;  // the direction is gathered next iteration
+    if (fabs(pq[0]) < DTINY) {
+      ierr = 2;
+      break;
+    }
+    const double al = rz / pq[0];
+    const double ax = al * rnorm0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = S.start + k * T + tid;
+      double c[1] = {0.0};
+      if (i < S.end) {
+        const double ri = fma(-al, qk[k], rs[i]);
+        begin_row(k, i, ri);
+        c[0] = ri * ri;
+      }
+      resident_put<1>(S.cp, S.cps, k, c);
+    }
+    if (!resident_exchange<WC, K>(S, z, a.st, [&] {
+#pragma unroll
+          for (int k = 0; k < K; ++k) {
+            const int i = S.start + k * T + tid;
+            if (i < S.end) a.x[i] = fma(ax, pk[k], a.x[i]);
+          }
+          total_post<1>(S, g);
+        }))
+      return;
+    double s2[1];
+    if (!total_wait<1>(S, g, a.st, s2)) return;
+    if (!(s2[0] <= stop2 || total >= a.maxit)) continue;
+    // r = b - A x in FP64 decides (the sum's barrier shows every block's x)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = S.start + k * T + tid;
+      double c[1] = {0.0};
+      if (i < S.end) {
+        const double ri = a.b[i] - row_spmv64<false>(a, a.x, i);
+        begin_row(k, i, ri * sc);
+        c[0] = ri * ri;
+      }
+      resident_put<1>(S.cp, S.cps, k, c);
+    }
+    if (!resident_exchange<WC, K>(S, z, a.st, [] {})) return;
+    double t2[1];
+    if (!resident_total<1>(S, g, a.st, t2)) return;  // x is written again only after every block has read it
+    rnorm = sqrt(t2[0]);
+    const double res = rnorm / bnrm;
+    if (res <= a.tol) {
+      write_result_m(a, g, total, res, 0);
+      return;
+    }
+    if (total >= a.maxit) {
+      ierr = 1;
+      break;
+    }
+    first = true;  // the recursive residual had drifted: restart from the true one
+  }
+  write_result_m(a, g, total, rnorm / bnrm, ierr);
+}
+
+// The block's part of the system: its range, its views and the prologue. False
+// when the kernel must leave (a wait ran out, or the result is already known:
+// b = 0, or a zero diagonal with code diag_code).
+template <int WC, int K, bool PCG>
+__device__ __forceinline__ bool resident_begin(const KrylovArgs& a, const MixedArgs& m, VGrid& g, Resident<WC>& S,
+                                               int R, int nhw_max, int diag_code, double& bnrm) {
+  const int n = a.n;
+  S.n = n;
+  S.R = R;
+  S.nb = g.nb;
+  S.start = g.rank * R;
+  S.end = min(n, S.start + R);
+  S.nsc = (n + kSuperRows - 1) / kSuperRows;
+  S.seq = S.rseq = 0u;
+  S.sums = m.red;
+  S.ll = reinterpret_cast<u64*>(m.w32);  // the FP32 work vectors' space
+  resident_views<WC>(S, R, m.plan.bw, nhw_max, K * (blockDim.x / 32));
+  bool diag_bad;
+  if (!resident_prologue<WC, K, PCG>(a, m, g, S, bnrm, diag_bad)) return false;
+  if (bnrm == 0.0) {
+    for (int i = S.start + threadIdx.x; i < S.end; i += blockDim.x) a.x[i] = 0.0;
+    write_result_m(a, g, 0, 0.0, 0);
+    return false;
+  }
+  if (diag_bad) {
+    write_result_m(a, g, 0, 0.0, diag_code);
+    return false;
+  }
+  return true;
+}
+
+// nhw_max: the halo words the shared memory was sized for.
+template <int WC, int K>
+__global__ void __launch_bounds__(kResidentThreads, 1) k_pcg_resident(KrylovArgs a, MixedArgs m, int R, int nhw_max) {
+  if (a.st->abort) return;
+  VGrid g = whole_grid(a.bar, a.partials, true);
+  const int T = blockDim.x, tid = threadIdx.x;
+  Resident<WC> S;
+  double bnrm;
+  if (!resident_begin<WC, K, true>(a, m, g, S, R, nhw_max, 2, bnrm)) return;
+  // Gershgorin bound of D^-1 A (a maximum is exact in any order), b - A x
+  double gm = 0.0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = S.start + k * T + tid;
+    double c[1] = {0.0};
+    if (i < S.end) {
+      double s = 0.0;
+      for (int q = a.row_ptr[i]; q < a.row_ptr[i + 1]; ++q) s += fabs(a.aval[q]);
+      gm = fmax(gm, s / fabs(a.aval[a.diag[i]]));
+      const double ri = a.b[i] - row_spmv64<false>(a, a.x, i);
+      a.r[i] = ri;
+      c[0] = ri * ri;
+    }
+    resident_put<1>(S.cp, S.cps, k, c);
+  }
+  if (!vg_max<false>(gm, g, a.st)) return;  // its barrier: nobody reads x any more
+  double rn[1];
+  if (!resident_total<1>(S, g, a.st, rn)) return;
+  const double rnorm = sqrt(rn[0]);
+  const double res = rnorm / bnrm;
+  if (res <= a.tol) {
+    write_result_m(a, g, 0, res, 0);
+    return;
+  }
+  const double lmax = gm, lmin = lmax / m.cheb_ratio;
+  const double th = 0.5 * (lmax + lmin);
+  if (tid == 0) {
+    const double de = 0.5 * (lmax - lmin), sg = th / de;
+    double rho0 = 1.0 / sg;
+    for (int j = 1; j < m.cheb_k; ++j) {
+      const double rho1 = 1.0 / (2.0 * sg - rho0);
+      s_cheb[j] = make_float2((float)(rho1 * rho0), (float)(2.0 * rho1 / de));
+      rho0 = rho1;
+    }
+  }
+  __syncthreads();
+  resident_pcg<WC, K>(a, m, g, S, bnrm, rnorm, (float)(1.0 / th));
+}
+
+// bicgstab_mixed_body (krylov_poly.cuh) on resident rows: the FP32 vectors in
+// registers, one exchange for each of the two products, the same recurrences,
+// sums and decisions.
+template <int WC, int K>
+__global__ void __launch_bounds__(kResidentThreads, 1) k_bicgstab_resident(KrylovArgs a, MixedArgs m, int R, int nhw_max) {
+  if (a.st->abort) return;
+  VGrid g = whole_grid(a.bar, a.partials, true);
+  const int T = blockDim.x, tid = threadIdx.x;
+  Resident<WC> S;
+  double bnrm;
+  if (!resident_begin<WC, K, false>(a, m, g, S, R, nhw_max, 12, bnrm)) return;
+  float r[K], r0[K], p[K], v[K], d[K];
+  int total = 0, ierr = 0;
+  double res = 0.0;
+  for (bool begun = false;; begun = true) {
+    // r = b - A x in FP64; the barrier shows every block's x
+    if (begun && !vg_sync(g, a.st)) return;
+    double w[1];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = S.start + k * T + tid;
+      double c[1] = {0.0};
+      if (i < S.end) {
+        const double ri = a.b[i] - row_spmv64<false>(a, a.x, i);
+        a.r[i] = ri;
+        c[0] = ri * ri;
+      }
+      resident_put<1>(S.cp, S.cps, k, c);
+    }
+    if (!resident_total<1>(S, g, a.st, w)) return;  // x is written again only after every block has read it
+    const double rnorm = sqrt(w[0]);
+    res = rnorm / bnrm;
+    if (res <= a.tol) {
+      write_result_m(a, g, total, res, 0);
+      return;
+    }
+    if (begun && total >= a.maxit) {
+      ierr = 1;
+      break;
+    }
+    const double inv = 1.0 / rnorm;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = S.start + k * T + tid;
+      r[k] = i < S.end ? (float)(a.r[i] * inv) : 0.0f;
+      r0[k] = r[k];
+      p[k] = v[k] = d[k] = 0.0f;
+      const double c[1] = {(double)r[k] * (double)r[k]};
+      resident_put<1>(S.cp, S.cps, k, c);
+    }
+    double w1[1];
+    if (!resident_total<1>(S, g, a.st, w1)) return;
+    const double target = m.tau * m.tau * w1[0];
+    double rho_next = w1[0], rho_old = 1.0, alpha = 1.0, omega = 1.0;
+    while (true) {
+      ++total;
+      const double rho = rho_next;
+      if (fabs(rho) < DTINY) {
+        ierr = 2;
+        break;
+      }
+      const float beta = (float)((rho / rho_old) * (alpha / omega));
+      const float om = (float)omega;
+      float e[K];  // the exchanged vector: ph = D^-1 p, then sh = D^-1 s
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int l = k * T + tid;
+        p[k] = fmaf(beta, fmaf(-om, v[k], p[k]), r[k]);
+        e[k] = l < S.R ? resident_dinv<WC>(S, l) * p[k] : 0.0f;
+      }
+      if (!resident_exchange<WC, K>(S, e, a.st, [] {})) return;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int l = k * T + tid;
+        float dinv;
+        v[k] = l < S.R ? resident_row<WC>(S, l, dinv) : 0.0f;
+        const double c[1] = {(double)r0[k] * (double)v[k]};
+        resident_put<1>(S.cp, S.cps, k, c);
+      }
+      double d1[1];
+      if (!resident_total<1>(S, g, a.st, d1)) return;
+      alpha = rho / d1[0];
+      const float af = (float)alpha;
+      // r becomes s; d takes the half step (its other half follows after omega)
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int l = k * T + tid;
+        d[k] = fmaf(af, e[k], d[k]);
+        r[k] = fmaf(-af, v[k], r[k]);
+        e[k] = l < S.R ? resident_dinv<WC>(S, l) * r[k] : 0.0f;
+        const double c[1] = {(double)r[k] * (double)r[k]};
+        resident_put<1>(S.cp, S.cps, k, c);
+      }
+      if (!resident_exchange<WC, K>(S, e, a.st, [&] { total_post<1>(S, g); })) return;
+      double d2[1];
+      if (!total_wait<1>(S, g, a.st, d2)) return;
+      if (d2[0] <= target || total >= a.maxit) break;
+      float t[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int l = k * T + tid;
+        float dinv;
+        t[k] = l < S.R ? resident_row<WC>(S, l, dinv) : 0.0f;
+        const double c[2] = {(double)t[k] * (double)t[k], (double)t[k] * (double)r[k]};
+        resident_put<2>(S.cp, S.cps, k, c);
+      }
+      double d3[2];
+      if (!resident_total<2>(S, g, a.st, d3)) return;
+      if (d3[0] < DTINY) {
+        ierr = 2;
+        break;
+      }
+      omega = d3[1] / d3[0];
+      if (fabs(omega) < DTINY) {
+        ierr = 2;
+        break;
+      }
+      const float omf = (float)omega;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        d[k] = fmaf(omf, e[k], d[k]);
+        r[k] = fmaf(-omf, t[k], r[k]);
+        const double c[2] = {(double)r[k] * (double)r[k], (double)r[k] * (double)r0[k]};
+        resident_put<2>(S.cp, S.cps, k, c);
+      }
+      double d4[2];
+      if (!resident_total<2>(S, g, a.st, d4)) return;
+      if (d4[0] <= target || total >= a.maxit) break;
+      rho_next = d4[1];
+      rho_old = rho;
+    }
+    if (ierr == 2) break;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = S.start + k * T + tid;
+      if (i < S.end) a.x[i] = fma(rnorm, (double)d[k], a.x[i]);
+    }
+  }
+  write_result_m(a, g, total, res, ierr);
+}
+
+// Halo words of the block of R rows at R * blockIdx.x: the 32-row words outside
+// its range that its columns touch; *most: the largest of all blocks. The
+// window's flags in dynamic shared memory.
+__global__ void k_halo_words(int n, int W, int ld, const int* __restrict__ ell_col, int bw, int R, int* most) {
+  extern __shared__ unsigned flags[];
+  const int s0 = blockIdx.x * R, e0 = s0 + R, wb = max(0, s0 - (bw + 31) / 32 * 32);
+  const int nwords = (min(n, e0 + bw) - wb + 31) / 32;
+  for (int w = threadIdx.x; w < nwords; w += blockDim.x) flags[w] = 0u;
+  __syncthreads();
+  for (int i = s0 + threadIdx.x; i < min(n, e0); i += blockDim.x)
+    for (int t = 0; t < W; ++t) {
+      const int c = ell_col[t * ld + i];
+      if (c < s0 || c >= e0) flags[(c - wb) >> 5] = 1u;
+    }
+  __syncthreads();
+  int mine = 0;
+  for (int w = threadIdx.x; w < nwords; w += blockDim.x) mine += flags[w] != 0u;
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  __shared__ int sum;
+  if (threadIdx.x == 0) sum = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicAdd(&sum, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(most, sum);
+}
+
+template <int WC>
+const void* resident_kernel(int K, bool pcg) {
+  switch (K) {
+    case 1: return pcg ? (const void*)k_pcg_resident<WC, 1> : (const void*)k_bicgstab_resident<WC, 1>;
+    case 2: return pcg ? (const void*)k_pcg_resident<WC, 2> : (const void*)k_bicgstab_resident<WC, 2>;
+    case 3: return pcg ? (const void*)k_pcg_resident<WC, 3> : (const void*)k_bicgstab_resident<WC, 3>;
+    case 4: return pcg ? (const void*)k_pcg_resident<WC, 4> : (const void*)k_bicgstab_resident<WC, 4>;
+    case 5: return pcg ? (const void*)k_pcg_resident<WC, 5> : (const void*)k_bicgstab_resident<WC, 5>;
+    case 7: return pcg ? (const void*)k_pcg_resident<WC, 7> : (const void*)k_bicgstab_resident<WC, 7>;
+    default: return pcg ? (const void*)k_pcg_resident<WC, 10> : (const void*)k_bicgstab_resident<WC, 10>;
+  }
+}
+
+constexpr int kStaticSmem = 2 * 1024;  // above the kernels' static shared memory and the driver's share of a block
+
+int device_limits(int& sms, int& smem_sm) {
+  int dev = 0;
+  MGPU_CUDA(cudaGetDevice(&dev));
+  MGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  MGPU_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  return 0;
+}
+
+// Threads of a block of R rows (a multiple of 256) and the rows of a thread,
+// one of the compiled counts.
+void resident_shape(int R, int& T, int& K) {
+  T = R >= kResidentThreads ? kResidentThreads : 256;
+  K = (R + T - 1) / T;
+  if (K > 5) K = K <= 7 ? 7 : 10;
+}
+
+}  // namespace
+
+// The division of a system over the SMs for its resident solves: rows of a
+// block (whole super-chunks) and the most halo words of a block; rows = 0 when
+// the system does not fit: the block's rows and window in an SM's shared
+// memory, window offsets in 16 bits, at most 7 entries a row.
+int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan& plan, cudaStream_t s) {
+  plan = ResidentPlan{};
+  if (!ell_col || W > 7 || bw < 0 || n < kSuperRows / 4) return 0;
+  int sms = 0, smem = 0;
+  if (int e = device_limits(sms, smem)) return e;
+  const int room = smem - kStaticSmem;
+  const int nsc = (n + kSuperRows - 1) / kSuperRows;
+  const int per = (nsc + sms - 1) / sms;
+  if (per > 20 || nsc > 2560) return 0;  // s_group holds 10 groups of 256 super-chunks
+  const int R = per * kSuperRows, WC = W <= 5 ? 5 : 7;
+  int T, K;
+  resident_shape(R, T, K);
+  const int flags = 4 * resident_window_words(R, bw);
+  if (resident_smem(WC, R, bw, 0, K * (T / 32)) > room || flags > 48 * 1024) return 0;
+  int* most = nullptr;
+  int h = 0;
+  MGPU_CUDA(cudaMallocAsync((void**)&most, sizeof(int), s));
+  MGPU_CUDA(cudaMemsetAsync(most, 0, sizeof(int), s));
+  k_halo_words<<<(nsc + per - 1) / per, 256, flags, s>>>(n, W, ld, ell_col, bw, R, most);
+  MGPU_CUDA(cudaGetLastError());
+  MGPU_CUDA(cudaMemcpyAsync(&h, most, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MGPU_CUDA(cudaFreeAsync(most, s));
+  MGPU_CUDA(cudaStreamSynchronize(s));
+  if (resident_smem(WC, R, bw, h, K * (T / 32)) > room || 4 * (R + 32 * h) > 65535) return 0;
+  plan.rows = R;
+  plan.words = h;
+  plan.bw = bw;
+  return 0;
+}
+
+// The resident solve of a planned system; *taken = false and no launch when
+// there is no plan or no polynomial to apply. A planned system always takes it:
+// from 64 rows (the smallest planned) to the largest that fits, about 570,000
+// rows of 7 entries, it measured faster than the streaming kernel.
+int launch_resident(const KrylovArgs& a, const MixedArgs& m, bool pcg, cudaStream_t s, bool* taken) {
+  *taken = false;
+  if (m.plan.rows <= 0 || (pcg && (!m.ell64 || m.cheb_k < 2 || m.cheb_k > 64))) return 0;
+  const int R = m.plan.rows, WC = m.ell_w <= 5 ? 5 : 7;
+  int T, K;
+  resident_shape(R, T, K);
+  const int dyn = resident_smem(WC, R, m.plan.bw, m.plan.words, K * (T / 32));
+  const void* fn = WC == 5 ? resident_kernel<5>(K, pcg) : resident_kernel<7>(K, pcg);
+  MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  KrylovArgs aa = a;
+  MixedArgs mm = m;
+  int RR = R, words = m.plan.words;
+  void* args[] = {&aa, &mm, &RR, &words};
+  MGPU_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
+  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3((a.n + R - 1) / R), dim3(T), args, (size_t)dyn, s));
+  *taken = true;
+  return 0;
+}
+
+}  // namespace mgpu

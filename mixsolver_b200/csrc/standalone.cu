@@ -146,7 +146,10 @@ int poly_solve(int n, const Pattern& P, const double* val, const double* b, doub
   int W = 0, *ell = nullptr;
   long ld = 0;
   TopoAlloc alloc = [&](int*& q, size_t k) { return B.alloc(q, k); };
-  TRY(device_ell(n, drp, dcol, 8, W, ld, ell, alloc, 0));
+  int bw = -1;  // the resident solve exchanges between blocks both ways: symmetric patterns only
+  TRY(device_ell(n, drp, dcol, 8, W, ld, ell, alloc, 0, &bw));
+  ResidentPlan plan;
+  if (sizeof(V) == 4 && P.symmetric) TRY(plan_resident(n, W, (int)ld, ell, bw, plan, 0));
   V* dev = nullptr;
   double* dev64 = nullptr;  // the mixed form's FP64 conjugate-gradient product
   if (ell) {
@@ -187,7 +190,7 @@ int poly_solve(int n, const Pattern& P, const double* val, const double* b, doub
   const double row_bytes = mixed ? mixed_row_bytes(W) : 16.0 * W + 80.0;
   const bool big = (double)n * row_bytes > g_prefetch_mb * 1048576.0;
   MixedArgsT<V> m{da,   ddinv, dw, 1e-4, cheb_degree, cheb_ratio, W, ell, dev, dred, (ell && big) ? 1 : 0, 0.0,
-                  (int)ld, 0,  dev64};
+                  (int)ld, 0,  dev64, plan};
   if constexpr (sizeof(V) == 4)
     TRY(launch_pcg_mixed(a, m, 0));
   else
