@@ -463,18 +463,16 @@ def run_ours(args):
         "accuracy": accuracy,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
-                     # DRAM bytes of one pressure-solve launch (36 iterations at the default
-                     # degree 24) from an ncu capture of this workload
-                     # (profiles/k_pcg_mixed_channel524k.md)
-                     "traffic": 1.914e9 if mixed and S.get_tuning("cheb_degree") == 24 else None,
-                     "resident": "L2: the system (~94 MB with its FP64 copy) stays in the 126 MB L2 across the "
-                                 "solve's passes, DRAM carries 5 % of the algorithmic bytes (ncu); frac is an "
-                                 "HBM-equivalent rate, see l2 for the fraction of the L2 roofline",
+                     "traffic": None,
+                     "resident": "shared memory: the FP32 matrix stays in the SMs' shared memory for the whole "
+                                 "solve and only the values that blocks exchange travel through L2; the "
+                                 "algorithmic bytes count it once a pass, so frac is an HBM-equivalent rate and "
+                                 "may exceed 1; see l2 for the fraction of the L2 roofline",
                      "l2": {"achieved": achieved, "peak": l2peak, "unit": "GB/s",
                             "frac": (achieved / l2peak) if achieved else None,
                             "peak_source": "L2-resident c = a + b over 3 x 16 MiB buffers, graph-replayed, "
                                            "measured in this run"},
-                     "kernel": "k_pcg_mixed (pressure solve)" if mixed else "k_factor+k_pcg (pressure solve)",
+                     "kernel": "k_pcg_resident (pressure solve)" if mixed else "k_factor+k_pcg (pressure solve)",
                      "algorithmic_bytes_per_launch": float(np.mean(ppe_bytes)), "avg_launch_ms": ppe_launch_ms,
                      "launches": len(ppe_ms), "all_krylov_solves_gbs": family,
                      "peak_source": peak_source},
@@ -544,9 +542,6 @@ def run_reference(args):
 
 
 PISO_METRIC = "PISO time steps/s, mixed vs FP64 GPU, rel L2 of u, p vs FP64"
-# DRAM bytes of the first corrector's pressure solve on the 3.07 M-tet box, by
-# Chebyshev degree, from ncu captures (profiles/k_pcg_mixed_piso3M.md)
-PISO_TRAFFIC = {24: 539.5e9, 48: 527.1e9}
 
 
 def run_piso(args):
@@ -664,13 +659,8 @@ def run_piso(args):
                    "rel_l2_vs_fp64": rel, "rel_l2_after_steps": args.fp64_steps},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
-                     # DRAM bytes of one pressure-solve launch (the first corrector) from
-                     # an ncu capture of this workload at the degree in effect
-                     # (profiles/k_pcg_mixed_piso3M.md)
-                     "traffic": PISO_TRAFFIC.get(S.get_tuning("cheb_degree_large")
-                                                 if 0 < S.get_tuning("cheb_large_rows") <= N
-                                                 else S.get_tuning("cheb_degree")),
-                     "kernel": "k_pcg_mixed (pressure solves)",
+                     "traffic": None,
+                     "kernel": "k_pcg_paged (pressure solves; k_pcg_resident up to about 820,000 tets)",
                      "algorithmic_bytes_per_launch": float(np.mean(ppe_bytes)), "avg_launch_ms": ppe_launch_ms,
                      "launches": len(ppe_ms), "all_krylov_solves_gbs": family,
                      "peak_source": peak_source},

@@ -24,6 +24,7 @@
 #include "mesh_host.h"
 
 namespace mgpu {
+size_t page_floats(int n, int W, const ResidentPlan& plan);  // krylov_resident.cu
 
 static thread_local std::string g_err;
 static int g_device = 0;
@@ -223,6 +224,8 @@ KrylovArgs base_args(MgpuCase* c) {
   a.st = d.st;
   a.recs = d.recs;
   a.ferr = d.ferr;
+  a.width = d.width;
+  a.bw = d.bw;
   a.tol = c->ctrl.lin_tol;
   a.maxit = c->ctrl.lin_max;
   return a;
@@ -669,9 +672,9 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
       (e = c->alloc(d.rhs, N)) || (e = c->alloc(d.pp, N)) || (e = c->alloc(d.uo, 3 * N)) ||
       (e = c->alloc(d.u_old, 3 * N)) || (e = c->alloc(d.u_old_old, 3 * N)) || (e = c->alloc(d.psi, N)) ||
       (e = c->alloc(d.af, F)) || (e = c->alloc(d.aval, d.nnz)) || (e = c->alloc(d.pval, d.nnz)) ||
-      (e = c->alloc(d.fval, d.nnz)) || (e = c->alloc(d.kw, 10 * N)) ||
+      (e = c->alloc(d.fval, d.nnz)) || (e = c->alloc(d.kw, (poly ? 10 : 16) * N)) ||
       (ctrl->precision == MGPU_PREC_MIXED &&
-       ((e = c->alloc(d.a32, d.nnz)) || (e = c->alloc(d.dinv32, N)) || (e = c->alloc(d.w32, 10 * N)))) ||
+       ((e = c->alloc(d.dinv32, N)) || (e = c->alloc(d.w32, 10 * N)))) ||
       (ctrl->precision == MGPU_PREC_FP64_POLY &&
        ((e = c->alloc(d.a64, d.nnz)) || (e = c->alloc(d.dinv64, N)) || (e = c->alloc(d.w64, 10 * N)))) ||
       (poly && (e = c->alloc(d.red32, (size_t)mixed_red_words(N)))) ||
@@ -684,6 +687,11 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
     MGPU_CUDA(cudaMemcpyAsync(d.ramp, one, sizeof(one), cudaMemcpyHostToDevice, c->stream));
   }
   if ((e = ensure_recs(c, 64))) return fail(e);
+  if (!poly) {
+    int wide = 0;
+    if ((e = device_row_extent(d.N, d.row_ptr, d.col, wide, d.bw, d.width, (int*)d.partials, c->stream)))
+      return fail(e);
+  }
   if (poly) {
     // column-major ELL copy of the pattern for the polynomial forms' SpMV (rows of at most 8 entries)
     int w = 0, bw = 0, *ell = nullptr;
@@ -699,11 +707,13 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
       if (ctrl->precision == MGPU_PREC_MIXED) {
         if ((e = c->alloc(d.ell_val, (size_t)w * ld))) return fail(e);
         MGPU_CUDA(cudaMemsetAsync(d.ell_val, 0, sizeof(float) * (size_t)w * ld, c->stream));
-        if ((e = plan_resident(d.N, w, (int)ld, ell, bw, d.plan, c->stream))) return fail(e);
+        if ((e = plan_resident(d.N, w, (int)ld, ell, bw, d.plan, d.ferr, c->stream))) return fail(e);
       }
       d.ell_w = w;
       d.ell_ld = (int)ld;
     }
+    // the pages of a larger system's pressure solve follow its CSR values
+    if (ctrl->precision == MGPU_PREC_MIXED && (e = c->alloc(d.a32, d.nnz + page_floats(d.N, w, d.plan)))) return fail(e);
   }
   // geometry (device), scratch for the node arrays and provisional centres
   std::vector<int> fptr_h(hm.fptr.begin(), hm.fptr.end());

@@ -43,7 +43,7 @@ struct KrylovArgs {
   double* fval;  // ILU(0)/IC(0) factor values (same pattern)
   const double* b;
   double* x;
-  double *r, *r0, *p, *v, *s, *t, *ph, *sh, *z, *w;
+  double *r, *r0, *p, *v, *s, *t, *ph, *sh, *z, *w;  // ten vectors in one array
   int nlev_lo;
   const int* lo_ptr;
   const int* lo_rows;
@@ -66,13 +66,18 @@ struct KrylovArgs {
   int* ferr;           // factorisation status written by the factor kernel
   int sweep_threads;   // threads of a sync-free triangular sweep (set at launch)
   int sweep_sleep;     // nanosleep of a long wait in that sweep (0: spin)
+  int width, bw;       // most entries of a row on one side of the diagonal (0: not known), largest |column - row|;
+                       // width > 0 also says that w is the last of ten work vectors in one array and 6 n more
+                       // doubles follow it
 };
 
 // How a system is divided for its resident solves (krylov_resident.cu): rows of
-// a block (0: the system does not fit), most 32-row words a block reads of
-// other blocks, largest |column - row|.
+// a block (0: no resident solve), most 32-row words a block reads of
+// other blocks, largest |column - row|; steps > 0: the system is larger than
+// the SMs' shared memory and its pressure solve takes the blocks in turns,
+// `steps` polynomial steps a turn.
 struct ResidentPlan {
-  int rows = 0, words = 0, bw = 0;
+  int rows = 0, words = 0, bw = 0, steps = 0;
 };
 
 // Data of a polynomial-preconditioned solve in working precision V: the
@@ -100,7 +105,7 @@ struct MixedArgsT {
   // the mixed form's PCG (V = float): the FP64 values in the ELL layout, for
   // the FP64 conjugate-gradient product q = A p (null: the CSR values)
   double* ell64;
-  ResidentPlan plan;  // krylov_resident.cu (rows 0: no resident solve)
+  ResidentPlan plan;  // krylov_resident.cu
 };
 using MixedArgs = MixedArgsT<float>;
 
@@ -154,6 +159,7 @@ struct LanePlan {
 
 struct DeviceCase {
   int N = 0, F = 0, nnz = 0;
+  int width = 0, bw = 0;  // FP64 form: most entries of a row on one side of the diagonal, largest |column - row|
   // faces
   int *c0 = nullptr, *c1 = nullptr, *fgrp = nullptr;
   double *xf = nullptr, *sf = nullptr, *area = nullptr, *lf = nullptr;  // xf,sf: 3 SoA planes
@@ -229,14 +235,15 @@ int launch_krylov_pcg(const KrylovArgs& a, cudaStream_t s);
 int launch_factor(const KrylovArgs& a, int kind, cudaStream_t s);
 int krylov_grid(int n, int& block, int which);
 int launch_pcg_mixed(const KrylovArgs& a, const MixedArgs& m, cudaStream_t s);
-// pattern symmetric, ell_col of W entries a row; waits for stream s
-int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan& plan, cudaStream_t s);
+// pattern symmetric, ell_col of W entries a row; scratch: one int on the device; waits for stream s
+int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan& plan, int* scratch, cudaStream_t s);
 int launch_resident(const KrylovArgs& a, const MixedArgs& m, bool pcg, cudaStream_t s, bool* taken);
 int launch_bicgstab_mixed(const KrylovArgs& a, const MixedArgs& m, cudaStream_t s);
 int launch_pcg_poly64(const KrylovArgs& a, const MixedArgsT<double>& m, cudaStream_t s);
 int launch_bicgstab_poly64(const KrylovArgs& a, const MixedArgsT<double>& m, cudaStream_t s);
 int batch_capacity(bool pcg, int ell);  // ell: 0 CSR, 1 ELL, 2 ELL + L2 prefetch
 int launch_mixed_batch(const LanePlan& p, bool pcg, int ell, cudaStream_t s);
+int launch_sweep(const KrylovArgs& a, bool pcg, cudaStream_t s, bool* taken);
 int launch_spmv(int n, const int* rp, const int* col, const double* val, const double* x, double* y,
                 cudaStream_t s);
 

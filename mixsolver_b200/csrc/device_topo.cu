@@ -363,20 +363,29 @@ __global__ void k_reverse(int N, const int* __restrict__ order, int* new_of_old)
 
 // ---------------- per-case lists ------------------------------------------
 
-// w[0]: the widest row; w[1]: the largest |column - row|
+// w[0]: the widest row; w[1]: the largest |column - row|; w[2]: the most entries
+// of a row on one side of the diagonal
 __global__ void k_row_width(int N, const int* __restrict__ rp, const int* __restrict__ col, int* w) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int wide = 0, far = 0;
+  int wide = 0, far = 0, side = 0;
   if (i < N) {
     const int b = rp[i], e = rp[i + 1];
     wide = e - b;
-    for (int k = b; k < e; ++k) far = max(far, abs(col[k] - i));
+    int lower = 0, upper = 0;
+    for (int k = b; k < e; ++k) {
+      far = max(far, abs(col[k] - i));
+      lower += col[k] < i;
+      upper += col[k] > i;
+    }
+    side = max(lower, upper);
   }
   wide = __reduce_max_sync(0xffffffffu, wide);
   far = __reduce_max_sync(0xffffffffu, far);
+  side = __reduce_max_sync(0xffffffffu, side);
   if ((threadIdx.x & 31) == 0) {
     atomicMax(w, wide);
     atomicMax(w + 1, far);
+    atomicMax(w + 2, side);
   }
 }
 
@@ -503,19 +512,26 @@ int device_topology(int N, int F, const int* c0, const int* c1, DeviceTopo& t, c
   return 0;
 }
 
+int device_row_extent(int N, const int* rp, const int* col, int& width, int& bw, int& side, int* w, cudaStream_t s) {
+  MGPU_CUDA(cudaMemsetAsync(w, 0, 3 * sizeof(int), s));
+  k_row_width<<<ceil_div(N, 256), 256, 0, s>>>(N, rp, col, w);
+  MGPU_LAUNCH_CHECK("k_row_width");
+  int h[3] = {0, 0, 0};
+  MGPU_CUDA(cudaMemcpyAsync(h, w, sizeof(h), cudaMemcpyDeviceToHost, s));
+  MGPU_CUDA(cudaStreamSynchronize(s));
+  width = h[0];
+  bw = h[1];
+  side = h[2];
+  return 0;
+}
+
 int device_ell(int N, const int* rp, const int* col, int max_width, int& W, long& ld, int*& ell,
                const TopoAlloc& alloc, cudaStream_t s, int* bandwidth) {
   Tmp T(s);
-  int* w = nullptr;
-  DT_TRY(T.get(w, 2));
-  MGPU_CUDA(cudaMemsetAsync(w, 0, 2 * sizeof(int), s));
-  k_row_width<<<ceil_div(N, 256), 256, 0, s>>>(N, rp, col, w);
-  MGPU_LAUNCH_CHECK("k_row_width");
-  int h[2] = {0, 0};
-  MGPU_CUDA(cudaMemcpyAsync(h, w, sizeof(h), cudaMemcpyDeviceToHost, s));
-  MGPU_CUDA(cudaStreamSynchronize(s));
-  W = h[0];
-  if (bandwidth) *bandwidth = h[1];
+  int *w = nullptr, bw = 0, side = 0;
+  DT_TRY(T.get(w, 3));
+  DT_TRY(device_row_extent(N, rp, col, W, bw, side, w, s));
+  if (bandwidth) *bandwidth = bw;
   ell = nullptr;
   ld = ((long)N + 3) / 4 * 4;  // each column starts on a 16-byte boundary
   if (W > max_width) return 0;

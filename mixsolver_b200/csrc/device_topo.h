@@ -28,6 +28,10 @@ using TopoAlloc = std::function<int(int*&, size_t)>;
 // nlev_lo = nlev_up = 0). Waits for stream s before returning.
 int device_topology(int N, int F, const int* c0, const int* c1, DeviceTopo& t, const TopoAlloc& alloc,
                     cudaStream_t s, bool levels = true);
+// Widest row, largest |column - row| and most entries of a row on one side of
+// the diagonal; scratch: three ints on the device. Waits for stream s.
+int device_row_extent(int N, const int* row_ptr, const int* col, int& width, int& bw, int& side, int* scratch,
+                      cudaStream_t s);
 // Widest row W of the pattern and, when W <= max_width, its column-major ELL
 // copy: entry t of row i at t * ld + i with ld = N rounded up to a multiple of
 // 4 (every column starts 16-byte aligned), padding the row itself.

@@ -66,7 +66,8 @@ __device__ __forceinline__ void resident_put(int cp, int cps, int k, const doubl
   }
 }
 
-__shared__ double s_group[2][2][10];  // group sums: parity, sum, group (a resident system has at most 10 groups)
+constexpr int kSumGroups = 64;  // groups of 256 super-chunks (65,536 rows) of a system, at most
+__shared__ double s_group[2][2][kSumGroups];  // group sums: half, sum, group
 
 // The group barrier in two halves, so that other work can run while the
 // arrivals travel: what the block wrote before arrive is visible to every
@@ -94,11 +95,13 @@ __device__ __forceinline__ bool vg_wait(VGrid& g, DevStatus* st) {
 // total_wait forms the total. The sums alternate between two halves: a block
 // writes sum s + 2 after the barrier of s + 1, at which every block has read
 // all of s.
+
+// The super-chunk sums of the state's rows (every thread; the chunk sums are
+// read only before the closing barrier of whoever puts the next ones).
 template <int NQ, typename State>
-__device__ __forceinline__ void total_post(State& S, const VGrid& g) {
+__device__ __forceinline__ void super_sums(const State& S) {
   constexpr int kChunks = kSuperRows / 32;
-  const unsigned seq = ++S.rseq;
-  double* sums = S.sums + (seq & 1u) * 2l * S.nsc;
+  double* sums = S.sums + (S.rseq & 1u) * 2l * S.nsc;
   __syncthreads();  // the chunk sums are written
   const int first = S.start / kSuperRows, mine = (S.end - S.start + kSuperRows - 1) / kSuperRows;
   for (int j = threadIdx.x; j < mine * NQ; j += blockDim.x) {
@@ -109,6 +112,12 @@ __device__ __forceinline__ void total_post(State& S, const VGrid& g) {
     for (int c = 1; c < kChunks; ++c) acc = acc + cq[c];
     sums[(long)q * S.nsc + first + b] = acc;
   }
+}
+
+template <int NQ, typename State>
+__device__ __forceinline__ void total_post(State& S, const VGrid& g) {
+  ++S.rseq;
+  super_sums<NQ>(S);
   vg_arrive(g);
 }
 

@@ -711,6 +711,9 @@ int krylov_grid(int n, int& block, int which) {
 }
 
 int launch_krylov_pcg(const KrylovArgs& a, cudaStream_t s) {
+  bool taken = false;  // factored systems that fit in the SMs' shared memory: krylov_sweep.cu
+  if (int e = launch_sweep(a, true, s, &taken)) return e;
+  if (taken) return 0;
   int block = 0;
   const int grid = krylov_grid(a.n, block, 0);
   KrylovArgs aa = a;
@@ -722,6 +725,9 @@ int launch_krylov_pcg(const KrylovArgs& a, cudaStream_t s) {
 }
 
 int launch_krylov_bicgstab(const KrylovArgs& a, cudaStream_t s) {
+  bool taken = false;
+  if (int e = launch_sweep(a, false, s, &taken)) return e;
+  if (taken) return 0;
   int block = 0;
   const int grid = krylov_grid(a.n, block, 1);
   KrylovArgs aa = a;

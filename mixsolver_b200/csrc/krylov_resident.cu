@@ -25,15 +25,15 @@
 // The sums keep the layout-independent tree of krylov_poly.cuh.
 //
 // Measured on a B200, one PCG iteration at degree 24 (streaming kernel ->
-// here): 6,400 rows 243 -> 32 us, 42,253 rows 99 -> 42 us, 82,944 rows (5
-// entries) 93 -> 42 us, 524,288 rows 181 -> 116 us; a BiCGStab iteration 42,253
+// here): 6,400 rows 243 -> 27 us, 42,253 rows 99 -> 35 us, 82,944 rows (5
+// entries) 93 -> 40 us, 524,288 rows 181 -> 116 us; a BiCGStab iteration 42,253
 // rows 24 -> 11 us, 524,288 rows 46 -> 33 us. A pass of the 524,288 rows is
 // 1.7 us of shared-memory reads (48 B of matrix and 7 gathers a row) and 1.9 us
-// of exchange. One block of 512 threads per SM: two blocks of 512 (64
-// registers each, one computing while the other's words travel) and one of
-// 1024 were 10-25 % slower, by their spills.
+// of exchange. Blocks of 512 threads two per SM and of 1024 (64 registers a
+// thread) were 10-25 % slower, by their spills.
 
 #include <algorithm>
+#include <cmath>
 
 #include "exchange.cuh"
 #include "krylov_poly.cuh"
@@ -41,7 +41,9 @@
 namespace mgpu {
 namespace {
 
-constexpr int kResidentThreads = 512;  // of a block, at most: 128 registers each
+// Blocks of 256 threads, two per SM, or of 512, one per SM; 128 registers each.
+constexpr int kResidentThreads = 512;
+constexpr int kPairRows = 9 * kSuperRows;  // rows of a block of 256 threads, at most
 constexpr int kHaloRegs = 4;   // halo words of a warp whose rows stay in registers
 constexpr int kHaloBatch = 16; // halo words of a warp whose polls are in flight together, at most
 
@@ -72,8 +74,18 @@ __host__ __device__ inline int resident_win_bytes(int R, int nhw, int wwin) {
   return ((win > scratch ? win : scratch) + 15) & ~15;
 }
 __host__ __device__ inline int resident_window_words(int R, int bw) { return R / 32 + 2 * ((bw + 31) / 32); }
+// matrix planes: values, then window offsets and the halo word list (its last
+// entry: their number, in a page)
+__host__ __device__ inline int resident_values(int WC, int R) { return (WC == 7 ? 32 : 24) * R; }
+__host__ __device__ inline int resident_places(int WC, int R, int nhw) {
+  return (WC == 7 ? 16 : 10) * R + ((2 * nhw + 2 + 15) & ~15);
+}
+// a page in global memory, whole lines
+__host__ __device__ inline int page_bytes(int WC, int R, int nhw) {
+  return (resident_values(WC, R) + resident_places(WC, R, nhw) + 127) & ~127;
+}
 __host__ __device__ inline int resident_smem(int WC, int R, int bw, int nhw, int cps) {
-  return resident_win_bytes(R, nhw, resident_window_words(R, bw)) + 16 * cps + (WC == 7 ? 48 : 34) * R + 2 * nhw;
+  return resident_win_bytes(R, nhw, resident_window_words(R, bw)) + 16 * cps + resident_values(WC, R) + resident_places(WC, R, nhw);
 }
 
 template <int WC>
@@ -186,26 +198,29 @@ __device__ __forceinline__ int halo_row(const Resident<WC>& S, int w) {
   return row < S.n ? row : own;
 }
 
-// One exchange: this block's new values z (registers) go to its exchange words
-// and its own window, the halo words are read until they carry this exchange's
-// number; between() runs while they travel. Words of the other parity may
-// still be read by a slower neighbour; these are free: a block writes exchange
-// s + 2 only after it has read the words s + 1 of every block it exchanges
-// with (the pattern is symmetric), which those wrote after reading all of
-// their words s. Returns false when a bounded poll ran out.
-template <int WC, int K, typename F>
-__device__ __forceinline__ bool resident_exchange(Resident<WC>& S, const float (&z)[K], DevStatus* st, F&& between) {
-  const int T = blockDim.x, tid = threadIdx.x, warp = tid >> 5, nw = T >> 5;
-  const unsigned seq = ++S.seq;
+// An exchange, number seq. Publish: this block's new values z (registers) to
+// its words. Receive: they go to its own window too, and the halo words are
+// read until they carry the number; the closing barrier also ends the reads of
+// the window before. Words of the other parity may still be read by a slower
+// neighbour; these are free: a block publishes exchange s + 2 only after it has
+// read the words s + 1 of every block it exchanges with (the pattern is
+// symmetric), which those published after reading all of their words s.
+// receive returns false when a bounded poll ran out.
+template <int WC, int K>
+__device__ __forceinline__ void resident_publish(const Resident<WC>& S, const float (&z)[K], unsigned seq) {
   u64* llb = S.ll + (long)(seq & 1u) * S.n;
-  if (S.nb > 1) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int i = S.start + k * T + tid;
-      if (i < S.end) st_word(llb + i, pack_word(__float_as_uint(z[k]), seq));
-    }
+  for (int k = 0; k < K; ++k) {
+    const int i = S.start + k * (int)blockDim.x + (int)threadIdx.x;
+    if (i < S.end) st_word(llb + i, pack_word(__float_as_uint(z[k]), seq));
   }
-  between();
+}
+
+template <int WC, int K>
+__device__ __forceinline__ bool resident_receive(const Resident<WC>& S, const float (&z)[K], unsigned seq,
+                                                 DevStatus* st) {
+  const int T = blockDim.x, tid = threadIdx.x, warp = tid >> 5, nw = T >> 5;
+  const u64* llb = S.ll + (long)(seq & 1u) * S.n;
   __syncthreads();  // the pass's reads of the window are done
 #pragma unroll
   for (int k = 0; k < K; ++k) {
@@ -239,14 +254,21 @@ __device__ __forceinline__ bool resident_exchange(Resident<WC>& S, const float (
   return __syncthreads_and(ok) != 0;
 }
 
-// The block's rows into shared memory: the window's halo words, ranked in
-// ascending order, the window offsets of the columns, the FP32 values and
-// inverse diagonals; the FP64 ELL values (PCG); the exchange words cleared
-// (the barrier puts every block's clears before the first exchange); b.b and
-// the count of zero diagonals.
+// The block's next exchange; between() runs while the words travel.
+template <int WC, int K, typename F>
+__device__ __forceinline__ bool resident_exchange(Resident<WC>& S, const float (&z)[K], DevStatus* st, F&& between) {
+  const unsigned seq = ++S.seq;
+  if (S.nb > 1) resident_publish<WC, K>(S, z, seq);
+  between();
+  return resident_receive<WC, K>(S, z, seq, st);
+}
+
+// The rows of the block's range into shared memory: the window's halo words,
+// ranked in ascending order, the window offsets of the columns, the FP32 values
+// and inverse diagonals; the FP64 ELL values (PCG); the exchange words cleared;
+// the chunk sums of b.b and of the zero diagonals.
 template <int WC, int K, bool PCG>
-__device__ __forceinline__ bool resident_prologue(const KrylovArgs& a, const MixedArgs& m, VGrid& g, Resident<WC>& S, double& bnrm,
-                                  bool& diag_bad) {
+__device__ __forceinline__ void resident_build(const KrylovArgs& a, const MixedArgs& m, Resident<WC>& S) {
   const int T = blockDim.x, tid = threadIdx.x, s0 = S.start, e0 = s0 + S.R;
   const int lane = tid & 31, warp = tid >> 5, nw = T >> 5;
   const int W = m.ell_w, ld = m.ell_ld;
@@ -337,6 +359,14 @@ __device__ __forceinline__ bool resident_prologue(const KrylovArgs& a, const Mix
     }
     resident_put<2>(S.cp, S.cps, k, c);
   }
+}
+
+// The block's rows, then b.b and the count of zero diagonals; the barrier puts
+// every block's cleared words before the first exchange.
+template <int WC, int K, bool PCG>
+__device__ __forceinline__ bool resident_prologue(const KrylovArgs& a, const MixedArgs& m, VGrid& g, Resident<WC>& S,
+                                                  double& bnrm, bool& diag_bad) {
+  resident_build<WC, K, PCG>(a, m, S);
   if (!vg_sync(g, a.st)) return false;
   double v[2];
   if (!resident_total<2>(S, g, a.st, v)) return false;
@@ -346,6 +376,23 @@ __device__ __forceinline__ bool resident_prologue(const KrylovArgs& a, const Mix
 }
 
 __shared__ float2 s_cheb[64];  // the polynomial's recurrence coefficients
+
+// cheb_apply's coefficients on [lmax / ratio, lmax] into s_cheb (every thread
+// calls it); returns 1 / theta of the first term.
+__device__ __forceinline__ float cheb_table(double lmax, double ratio, int degree) {
+  const double lmin = lmax / ratio;
+  const double th = 0.5 * (lmax + lmin), de = 0.5 * (lmax - lmin), sg = th / de;
+  if (threadIdx.x == 0) {
+    double rho0 = 1.0 / sg;
+    for (int j = 1; j < degree; ++j) {
+      const double rho1 = 1.0 / (2.0 * sg - rho0);
+      s_cheb[j] = make_float2((float)(rho1 * rho0), (float)(2.0 * rho1 / de));
+      rho0 = rho1;
+    }
+  }
+  __syncthreads();
+  return (float)(1.0 / th);
+}
 
 // The Chebyshev-Jacobi polynomial of cheb_apply on the block's rows: on entry
 // z holds z0 (registers, exchanged); on return z is the result, exchanged, and
@@ -594,20 +641,344 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_pcg_resident(KrylovArgs
     write_result_m(a, g, 0, res, 0);
     return;
   }
-  const double lmax = gm, lmin = lmax / m.cheb_ratio;
-  const double th = 0.5 * (lmax + lmin);
-  if (tid == 0) {
-    const double de = 0.5 * (lmax - lmin), sg = th / de;
-    double rho0 = 1.0 / sg;
-    for (int j = 1; j < m.cheb_k; ++j) {
-      const double rho1 = 1.0 / (2.0 * sg - rho0);
-      s_cheb[j] = make_float2((float)(rho1 * rho0), (float)(2.0 * rho1 / de));
-      rho0 = rho1;
+  const float inv_th = cheb_table(gm, m.cheb_ratio, m.cheb_k);
+  resident_pcg<WC, K>(a, m, g, S, bnrm, rnorm, inv_th);
+}
+
+// ---------------------------------------------------------------------------
+// Larger systems: the blocks' rows in turns
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// The PCG of resident_pcg for a system larger than the SMs' shared memory. What
+// bounds it when streamed (k_pcg_mixed) is the matrix: every Chebyshev pass
+// reads all of it, 40 or 56 bytes a row, from HBM. Here the rows are cut into
+// pages (what a resident block holds: planes of matrix rows, window offsets and
+// halo words, built once a solve in global memory). Block b takes pages b, b +
+// nb, ... in turn, loads one into shared memory and runs plan.steps polynomial
+// steps on it before the next, exchanging values step by step with the blocks
+// that hold the neighbouring pages, so the matrix is read once per plan.steps
+// passes. There is no barrier: page p's step s waits for the words of step
+// s - 1 of the pages its rows refer to, at most r = ceil(bw / rows) pages
+// ahead. No wait is circular: within a sweep over the pages, order the steps
+// by (p + s r); a step waits for words of lesser or equal rank and lesser s,
+// and a block's turn at page p + nb starts after its last step at p, of rank
+// p + steps r < p + nb + r while (steps - 1) r < nb (the plan keeps to half of
+// that); a sweep never waits for a later one. The other vectors stream.
+// Measured on a B200, a solve streamed -> here: 2,000,376 rows of 7 entries, 35
+// iterations at degree 48, 54.2 -> 46.4 ms; 3,072,000 rows of 5, 53 iterations,
+// 100.3 -> 96.4 ms. A step of a page takes 1.7 us of shared-memory reads and 2.9 us
+// of exchange (1.9 in the resident solve: here L2 also carries the pages), a turn
+// 4.8 us to load.
+template <int WC, int K>
+__global__ void __launch_bounds__(256, 2) k_pcg_paged(KrylovArgs a, MixedArgs m) {
+  if (a.st->abort) return;
+  VGrid g = whole_grid(a.bar, a.partials, true);
+  const int n = a.n, T = blockDim.x, tid = threadIdx.x, R = m.plan.rows, W = m.ell_w, ld = m.ell_ld;
+  const int npages = (n + R - 1) / R, degree = m.cheb_k;
+  const int vbytes = resident_values(WC, R), pb = vbytes + resident_places(WC, R, m.plan.words);
+  const long pstep = page_bytes(WC, R, m.plan.words);
+  const int warp = tid >> 5, nw = T >> 5;
+  Resident<WC> S;
+  S.n = n;
+  S.R = R;
+  S.nb = npages;
+  S.nsc = (n + kSuperRows - 1) / kSuperRows;
+  S.seq = S.rseq = 0u;
+  S.sums = m.red;
+  S.ll = reinterpret_cast<u64*>(m.w32);
+  float *dch = m.w32 + 4l * n, *rr = m.w32 + 5l * n, *zf = m.w32 + 6l * n;
+  resident_views<WC>(S, R, m.plan.bw, m.plan.words, K * (T / 32));
+  // the pages follow the FP32 CSR values
+  unsigned char* const pages = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<unsigned long long>(m.a32 + a.row_ptr[n]) + 127) & ~127ull);
+  auto turn = [&](int p) {
+    S.start = p * R;
+    S.end = min(n, S.start + R);
+    S.wb = max(0, S.start - (m.plan.bw + 31) / 32 * 32);
+  };
+// a page's rows, in tiles of T
+#define MGPU_PAGE_ROWS(k, i) \
+  for (int k = 0; k < K; ++k) \
+    if (const int i = S.start + k * T + tid; true)
+  // the pages, b.b, the zero diagonals
+  double gm = 0.0;
+  ++S.rseq;
+  for (int p = g.rank; p < npages; p += g.nb) {
+    turn(p);
+    __syncthreads();  // the page before has left shared memory
+    resident_build<WC, K, true>(a, m, S);
+    if (tid == 0) smem_at<unsigned short>(S.words, m.plan.words) = (unsigned short)S.nhw;
+    MGPU_PAGE_ROWS(k, i) {
+      if (i < S.end) {
+        m.dinv[i] = resident_dinv<WC>(S, k * T + tid);
+        double s = 0.0;
+        for (int q = a.row_ptr[i]; q < a.row_ptr[i + 1]; ++q) s += fabs(a.aval[q]);
+        gm = fmax(gm, s / fabs(a.aval[a.diag[i]]));
+      }
+    }
+    super_sums<2>(S);
+    uint4* page = reinterpret_cast<uint4*>(pages + p * pstep);
+    for (int o = tid; o < pb / 16; o += T) page[o] = smem_at<uint4>(S.va, o);
+  }
+  vg_arrive(g);
+  double v2[2];
+  if (!total_wait<2>(S, g, a.st, v2)) return;
+  const double bnrm = sqrt(v2[0]);
+  if (bnrm == 0.0) {
+    for (int p = g.rank; p < npages; p += g.nb) {
+      turn(p);
+      MGPU_PAGE_ROWS(k, i) {
+        if (i < S.end) a.x[i] = 0.0;
+      }
+    }
+    write_result_m(a, g, 0, 0.0, 0);
+    return;
+  }
+  if (v2[1] != 0.0) {
+    write_result_m(a, g, 0, 0.0, 2);
+    return;
+  }
+  // r = b - A x
+  ++S.rseq;
+  for (int p = g.rank; p < npages; p += g.nb) {
+    turn(p);
+    __syncthreads();
+    MGPU_PAGE_ROWS(k, i) {
+      double c[1] = {0.0};
+      if (i < S.end) {
+        const double ri = a.b[i] - row_spmv64<false>(a, a.x, i);
+        a.r[i] = ri;
+        c[0] = ri * ri;
+      }
+      resident_put<1>(S.cp, S.cps, k, c);
+    }
+    super_sums<1>(S);
+  }
+  if (!vg_max<false>(gm, g, a.st)) return;
+  vg_arrive(g);
+  double t1[1];
+  if (!total_wait<1>(S, g, a.st, t1)) return;
+  const double rnorm0 = sqrt(t1[0]);
+  double res = rnorm0 / bnrm, rnorm = rnorm0;
+  if (res <= a.tol) {
+    write_result_m(a, g, 0, res, 0);
+    return;
+  }
+  const float inv_th = cheb_table(gm, m.cheb_ratio, degree);
+  double *rs = a.r, *pd = a.p, *pn = a.s, *qd = a.v;
+  const double* __restrict__ ev = m.ell64;
+  const int* __restrict__ ecol = m.ell_col;
+  const float* __restrict__ dinv = m.dinv;
+  const double sc = 1.0 / rnorm0, stop = a.tol * bnrm * sc, stop2 = stop * stop;
+  // row i of the scaled residual: its FP32 copy, the first Chebyshev term, which
+  // is published as exchange S.seq
+  auto begin_row = [&](int i, double ri) {
+    rs[i] = ri;
+    const float rf = (float)ri;
+    rr[i] = rf;
+    const float z0 = dinv[i] * rf * inv_th;
+    dch[i] = z0;
+    st_word(S.ll + (long)(S.seq & 1u) * n + i, pack_word(__float_as_uint(z0), S.seq));
+  };
+  ++S.seq;
+  for (int p = g.rank; p < npages; p += g.nb) {
+    turn(p);
+    MGPU_PAGE_ROWS(k, i) {
+      if (i < S.end) begin_row(i, a.r[i] * sc);
     }
   }
-  __syncthreads();
-  resident_pcg<WC, K>(a, m, g, S, bnrm, rnorm, (float)(1.0 / th));
+  double rz = 0.0;
+  int total = 0, ierr = 0;
+  bool first = true;
+  while (true) {
+    // the polynomial: sweeps of up to plan.steps steps a page
+    ++S.rseq;
+    for (int done = 0; done < degree - 1;) {
+      const int ns = min(m.plan.steps, degree - 1 - done);
+      const bool final = done + ns == degree - 1;
+      for (int p = g.rank; p < npages; p += g.nb) {
+        turn(p);
+        __syncthreads();  // the page before has left shared memory
+        const unsigned char* page = pages + p * pstep;
+        for (int o = 16 * tid; o < pb; o += 16 * T) cp_async16(block_smem + S.va + o, page + o);
+        float z[K], d[K], rv[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const int i = S.start + k * T + tid;
+          z[k] = d[k] = rv[k] = 0.0f;
+          if (i < S.end) {
+            z[k] = __uint_as_float((unsigned)ld_word(S.ll + (long)(S.seq & 1u) * n + i));
+            d[k] = dch[i];
+            rv[k] = rr[i];
+          }
+        }
+        // the block's next page on its way to L2 while this one is at work
+        {
+          const int pnext = p + g.nb < npages ? p + g.nb : g.rank;
+          const unsigned char* next = pages + pnext * pstep;
+          for (int o = 128 * tid; o < pb; o += 128 * T) prefetch_l2(next + o);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        S.nhw = smem_at<unsigned short>(S.words, m.plan.words);
+        S.hpw = (S.nhw + nw - 1) / nw;
+#pragma unroll
+        for (int q = 0; q < kHaloRegs; ++q) S.hrow[q] = halo_row(S, warp + q * nw);
+        for (int j = 1; j <= ns; ++j) {
+          if (!resident_receive<WC, K>(S, z, S.seq + j - 1, a.st)) return;
+          const float2 c = s_cheb[done + j];
+#pragma unroll
+          for (int k = 0; k < K; ++k) {
+            const int l = k * T + tid;
+            if (l < R) {
+              float di;
+              const float az = resident_row<WC>(S, l, di);
+              const float rk = di * (rv[k] - az);
+              d[k] = fmaf(c.x, d[k], c.y * rk);
+              z[k] = z[k] + d[k];
+            }
+          }
+          resident_publish<WC, K>(S, z, S.seq + j);
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const int i = S.start + k * T + tid;
+          double c[1] = {0.0};
+          if (i < S.end) {
+            if (final) {
+              zf[i] = z[k];
+              c[0] = rs[i] * (double)z[k];
+            } else {
+              dch[i] = d[k];
+            }
+          }
+          if (final) resident_put<1>(S.cp, S.cps, k, c);
+        }
+        if (final) super_sums<1>(S);
+      }
+      S.seq += ns;
+      done += ns;
+    }
+    vg_arrive(g);
+    if (!total_wait<1>(S, g, a.st, t1)) return;
+    const double rzn = t1[0];
+    double beta = 0.0;
+    if (!first) {
+      if (fabs(rz) < DTINY) {
+        ierr = 2;
+        break;
+      }
+      beta = rzn / rz;
+    }
+    rz = rzn;
+    ++total;
+    // pn := z + beta p, q := A pn
+    ++S.rseq;
+    for (int p = g.rank; p < npages; p += g.nb) {
+      turn(p);
+      __syncthreads();
+#pragma unroll 2
+      MGPU_PAGE_ROWS(k, i) {
+        double c[1] = {0.0};
+        if (i < S.end) {
+          double v[WC], x[WC];
+          int cc[WC];
+#pragma unroll
+          for (int t = 0; t < WC; ++t)
+            if (t < W) {
+              cc[t] = ecol[t * ld + i];
+              v[t] = ev[t * ld + i];
+            }
+#pragma unroll
+          for (int t = 0; t < WC; ++t)
+            if (t < W) x[t] = first ? (double)ldv(&zf[cc[t]]) : fma(beta, ldv(&pd[cc[t]]), (double)ldv(&zf[cc[t]]));
+          double acc = 0.0;
+#pragma unroll
+          for (int t = 0; t < WC; ++t)
+            if (t < W) acc = fma(v[t], x[t], acc);
+          const double pi = first ? (double)zf[i] : fma(beta, pd[i], (double)zf[i]);
+          pn[i] = pi;
+          qd[i] = acc;
+          c[0] = pi * acc;
+        }
+        resident_put<1>(S.cp, S.cps, k, c);
+      }
+      super_sums<1>(S);
+    }
+    {
+      double* t = pd;
+      pd = pn;
+      pn = t;
+    }
+    first = false;
+    vg_arrive(g);
+    if (!total_wait<1>(S, g, a.st, t1)) return;
+    if (fabs(t1[0]) < DTINY) {
+      ierr = 2;
+      break;
+    }
+    const double al = rz / t1[0];
+    const double ax = al * rnorm0;
+    ++S.rseq;
+    ++S.seq;
+    for (int p = g.rank; p < npages; p += g.nb) {
+      turn(p);
+      __syncthreads();
+#pragma unroll 2
+      MGPU_PAGE_ROWS(k, i) {
+        double c[1] = {0.0};
+        if (i < S.end) {
+          a.x[i] = fma(ax, pd[i], a.x[i]);
+          const double ri = fma(-al, qd[i], rs[i]);
+          begin_row(i, ri);
+          c[0] = ri * ri;
+        }
+        resident_put<1>(S.cp, S.cps, k, c);
+      }
+      super_sums<1>(S);
+    }
+    vg_arrive(g);
+    if (!total_wait<1>(S, g, a.st, t1)) return;
+    if (!(t1[0] <= stop2 || total >= a.maxit)) continue;
+    // r = b - A x in FP64 decides
+    ++S.rseq;
+    ++S.seq;
+    for (int p = g.rank; p < npages; p += g.nb) {
+      turn(p);
+      __syncthreads();
+      MGPU_PAGE_ROWS(k, i) {
+        double c[1] = {0.0};
+        if (i < S.end) {
+          const double ri = a.b[i] - row_spmv64<false>(a, a.x, i);
+          begin_row(i, ri * sc);
+          c[0] = ri * ri;
+        }
+        resident_put<1>(S.cp, S.cps, k, c);
+      }
+      super_sums<1>(S);
+    }
+    vg_arrive(g);
+    if (!total_wait<1>(S, g, a.st, t1)) return;
+    rnorm = sqrt(t1[0]);
+    res = rnorm / bnrm;
+    if (res <= a.tol) {
+      write_result_m(a, g, total, res, 0);
+      return;
+    }
+    if (total >= a.maxit) {
+      ierr = 1;
+      break;
+    }
+    first = true;
+  }
+  write_result_m(a, g, total, rnorm / bnrm, ierr);
 }
+#undef MGPU_PAGE_ROWS
 
 // bicgstab_mixed_body (krylov_poly.cuh) on resident rows: the FP32 vectors in
 // registers, one exchange for each of the two products, the same recurrences,
@@ -776,92 +1147,163 @@ __global__ void k_halo_words(int n, int W, int ld, const int* __restrict__ ell_c
   if (threadIdx.x == 0) atomicMax(most, sum);
 }
 
+enum { kBicg = 0, kPcg = 1, kPcgPaged = 2 };
+
+template <int WC, int K>
+const void* resident_kernel_k(int which) {
+  if constexpr (K >= 7)
+    if (which == kPcgPaged) return (const void*)k_pcg_paged<WC, K>;
+  return which == kPcg ? (const void*)k_pcg_resident<WC, K> : (const void*)k_bicgstab_resident<WC, K>;
+}
+
 template <int WC>
-const void* resident_kernel(int K, bool pcg) {
+const void* resident_kernel(int K, int which) {
   switch (K) {
-    case 1: return pcg ? (const void*)k_pcg_resident<WC, 1> : (const void*)k_bicgstab_resident<WC, 1>;
-    case 2: return pcg ? (const void*)k_pcg_resident<WC, 2> : (const void*)k_bicgstab_resident<WC, 2>;
-    case 3: return pcg ? (const void*)k_pcg_resident<WC, 3> : (const void*)k_bicgstab_resident<WC, 3>;
-    case 4: return pcg ? (const void*)k_pcg_resident<WC, 4> : (const void*)k_bicgstab_resident<WC, 4>;
-    case 5: return pcg ? (const void*)k_pcg_resident<WC, 5> : (const void*)k_bicgstab_resident<WC, 5>;
-    case 7: return pcg ? (const void*)k_pcg_resident<WC, 7> : (const void*)k_bicgstab_resident<WC, 7>;
-    default: return pcg ? (const void*)k_pcg_resident<WC, 10> : (const void*)k_bicgstab_resident<WC, 10>;
+    case 1: return resident_kernel_k<WC, 1>(which);
+    case 2: return resident_kernel_k<WC, 2>(which);
+    case 3: return resident_kernel_k<WC, 3>(which);
+    case 4: return resident_kernel_k<WC, 4>(which);
+    case 5: return resident_kernel_k<WC, 5>(which);
+    case 7: return resident_kernel_k<WC, 7>(which);
+    default: return resident_kernel_k<WC, 9>(which);
   }
 }
 
-constexpr int kStaticSmem = 2 * 1024;  // above the kernels' static shared memory and the driver's share of a block
+constexpr int kStaticSmem = 4 * 1024;  // above the kernels' static shared memory and the driver's share of a block
 
 int device_limits(int& sms, int& smem_sm) {
   int dev = 0;
   MGPU_CUDA(cudaGetDevice(&dev));
   MGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  MGPU_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  MGPU_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
   return 0;
 }
 
 // Threads of a block of R rows (a multiple of 256) and the rows of a thread,
 // one of the compiled counts.
 void resident_shape(int R, int& T, int& K) {
-  T = R >= kResidentThreads ? kResidentThreads : 256;
+  T = R > kPairRows ? 512 : 256;
   K = (R + T - 1) / T;
-  if (K > 5) K = K <= 7 ? 7 : 10;
+  if (K > 5) K = K <= 7 ? 7 : 9;
 }
 
 }  // namespace
 
+namespace {
+// The most halo words of a block when the rows are cut into blocks of R, and
+// whether such a block fits: rows and window in an SM's shared memory, window
+// offsets in 16 bits.
+int fit_rows(int n, int W, int ld, const int* ell_col, int bw, int R, int room, int& words, bool& fits, int* most,
+             cudaStream_t s) {
+  const int WC = W <= 5 ? 5 : 7, flags = 4 * resident_window_words(R, bw);
+  int T, K;
+  resident_shape(R, T, K);
+  fits = false;
+  if (resident_smem(WC, R, bw, 0, K * (T / 32)) > room || flags > 48 * 1024) return 0;
+  MGPU_CUDA(cudaMemsetAsync(most, 0, sizeof(int), s));
+  k_halo_words<<<(n + R - 1) / R, 256, flags, s>>>(n, W, ld, ell_col, bw, R, most);
+  MGPU_CUDA(cudaGetLastError());
+  MGPU_CUDA(cudaMemcpyAsync(&words, most, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MGPU_CUDA(cudaStreamSynchronize(s));
+  fits = resident_smem(WC, R, bw, words, K * (T / 32)) <= room && 4 * (R + 32 * words) <= 65535;
+  return 0;
+}
+}  // namespace
+
 // The division of a system over the SMs for its resident solves: rows of a
-// block (whole super-chunks) and the most halo words of a block; rows = 0 when
-// the system does not fit: the block's rows and window in an SM's shared
-// memory, window offsets in 16 bits, at most 7 entries a row.
-int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan& plan, cudaStream_t s) {
+// block (whole super-chunks) and the most halo words of a block; larger systems:
+// the largest page and the steps of its turn. No plan (rows 0) with more than 7
+// entries a row, or when the halo does not fit.
+int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan& plan, int* scratch, cudaStream_t s) {
   plan = ResidentPlan{};
   if (!ell_col || W > 7 || bw < 0 || n < kSuperRows / 4) return 0;
   int sms = 0, smem = 0;
   if (int e = device_limits(sms, smem)) return e;
-  const int room = smem - kStaticSmem;
   const int nsc = (n + kSuperRows - 1) / kSuperRows;
-  const int per = (nsc + sms - 1) / sms;
-  if (per > 20 || nsc > 2560) return 0;  // s_group holds 10 groups of 256 super-chunks
-  const int R = per * kSuperRows, WC = W <= 5 ? 5 : 7;
-  int T, K;
-  resident_shape(R, T, K);
-  const int flags = 4 * resident_window_words(R, bw);
-  if (resident_smem(WC, R, bw, 0, K * (T / 32)) > room || flags > 48 * 1024) return 0;
-  int* most = nullptr;
-  int h = 0;
-  MGPU_CUDA(cudaMallocAsync((void**)&most, sizeof(int), s));
-  MGPU_CUDA(cudaMemsetAsync(most, 0, sizeof(int), s));
-  k_halo_words<<<(nsc + per - 1) / per, 256, flags, s>>>(n, W, ld, ell_col, bw, R, most);
-  MGPU_CUDA(cudaGetLastError());
-  MGPU_CUDA(cudaMemcpyAsync(&h, most, sizeof(int), cudaMemcpyDeviceToHost, s));
-  MGPU_CUDA(cudaFreeAsync(most, s));
-  MGPU_CUDA(cudaStreamSynchronize(s));
-  if (resident_smem(WC, R, bw, h, K * (T / 32)) > room || 4 * (R + 32 * h) > 65535) return 0;
-  plan.rows = R;
-  plan.words = h;
-  plan.bw = bw;
+  if (nsc > 256 * kSumGroups) return 0;
+  const int pair = (nsc + 2 * sms - 1) / (2 * sms), single = (nsc + sms - 1) / sms;
+  const int half = smem / 2 - kStaticSmem, whole = smem - kStaticSmem;
+  int words = 0;
+  bool fits = false;
+  auto keep = [&](int R) {
+    plan.rows = R;
+    plan.words = words;
+    plan.bw = bw;
+  };
+  // two blocks of 256 threads per SM up to 6 super-chunks each (one PCG
+  // iteration of 42,253 rows 42 -> 35 us against one block of 512), then one of
+  // 512 (524,288 rows: 116 us against 121 for two of 256)
+  if (pair <= 6) {
+    if (int e = fit_rows(n, W, ld, ell_col, bw, pair * kSuperRows, half, words, fits, scratch, s)) return e;
+    if (fits) keep(pair * kSuperRows);
+    if (fits) return 0;
+  }
+  if (single * kSuperRows > kPairRows && single <= 18) {
+    if (int e = fit_rows(n, W, ld, ell_col, bw, single * kSuperRows, whole, words, fits, scratch, s)) return e;
+    if (fits) keep(single * kSuperRows);
+    if (fits) return 0;
+  }
+  // pages: the largest that fits in half an SM, and the steps that make the most
+  // of the shared memory. With G blocks, r pages of reach and a load that takes as
+  // long as L steps, steps pass at s (G - (s - 1) r) / (L + s) pages a step time
+  // (each page waits (s - 1) r pages' worth for those ahead of it). L = 2 fits a
+  // B200 (3,072,000 rows, r = 5.2: 111, 102, 96, 94 ms at 3, 5, 8, 10 steps); the
+  // streamed pass took about 2.3 G page-step times, so the turns are used while
+  // they promise a fifth less than that.
+  const int most = 2 * sms;
+  for (int sc = 9; sc >= 5 && !fits; --sc) {
+    const int R = sc * kSuperRows;
+    if (R * (long)most > n) continue;  // a page for every block at least
+    if (int e = fit_rows(n, W, ld, ell_col, bw, R, half, words, fits, scratch, s)) return e;
+    if (!fits) continue;
+    const double r = (double)bw / R;
+    double best = 0.0;
+    for (int st = 2; st <= 16 && 2 * (st - 1) * (int)std::ceil(r) < most; ++st) {
+      const double rate = st * (most - (st - 1) * r) / (2.0 + st);
+      if (rate > best) {
+        best = rate;
+        plan.steps = st;
+      }
+    }
+    if (best <= 0.0 || most / best > 0.8 * 2.3) {
+      plan = ResidentPlan{};
+      return 0;
+    }
+    keep(R);
+  }
   return 0;
 }
 
+// Floats that a plan's pages take after the FP32 CSR values (MixedArgs::a32).
+size_t page_floats(int n, int W, const ResidentPlan& plan) {
+  if (plan.steps == 0) return 0;
+  return (size_t)page_bytes(W <= 5 ? 5 : 7, plan.rows, plan.words) / 4 * ((n + plan.rows - 1) / plan.rows) + 32;
+}
+
 // The resident solve of a planned system; *taken = false and no launch when
-// there is no plan or no polynomial to apply. A planned system always takes it:
-// from 64 rows (the smallest planned) to the largest that fits, about 570,000
-// rows of 7 entries, it measured faster than the streaming kernel.
+// there is no plan, no polynomial to apply, or turns are planned (pressure only). A planned system always takes it: from 64 rows (the smallest
+// planned) to the largest that fits, about 570,000 rows of 7 entries, it measured
+// faster than the streaming kernel.
 int launch_resident(const KrylovArgs& a, const MixedArgs& m, bool pcg, cudaStream_t s, bool* taken) {
   *taken = false;
   if (m.plan.rows <= 0 || (pcg && (!m.ell64 || m.cheb_k < 2 || m.cheb_k > 64))) return 0;
+  const bool paged = m.plan.steps > 0;
+  if (paged && !pcg) return 0;
   const int R = m.plan.rows, WC = m.ell_w <= 5 ? 5 : 7;
-  int T, K;
+  int T, K, sms = 0, smem = 0;
+  if (int e = device_limits(sms, smem)) return e;
   resident_shape(R, T, K);
   const int dyn = resident_smem(WC, R, m.plan.bw, m.plan.words, K * (T / 32));
-  const void* fn = WC == 5 ? resident_kernel<5>(K, pcg) : resident_kernel<7>(K, pcg);
+  const int which = paged ? kPcgPaged : pcg ? kPcg : kBicg;
+  const void* fn = WC == 5 ? resident_kernel<5>(K, which) : resident_kernel<7>(K, which);
   MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   KrylovArgs aa = a;
   MixedArgs mm = m;
   int RR = R, words = m.plan.words;
-  void* args[] = {&aa, &mm, &RR, &words};
+  void* args[] = {&aa, &mm, &RR, &words};  // the paged kernel takes the first two
+  const int grid = std::min((a.n + R - 1) / R, paged ? 2 * sms : 1 << 30);
   MGPU_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
-  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3((a.n + R - 1) / R), dim3(T), args, (size_t)dyn, s));
+  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(T), args, (size_t)dyn, s));
   *taken = true;
   return 0;
 }

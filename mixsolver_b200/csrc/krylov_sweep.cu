@@ -1,22 +1,34 @@
 // krylov_sweep.cu -- the FP64 parity form's ILU(0) / IC(0) solves on rows that
 // stay in shared memory: cg_ic0 and PCG+ILU(0), bicgstab_ilu0
-// (mod_uns_linsolver.f90:148-224, 405-461), with the row arithmetic and order of
-// krylov.cu.
+// (mod_uns_linsolver.f90:148-224, 405-461), the same bits as krylov.cu's.
 //
 // What bounds these solves is the serial chain of the triangular sweeps: one hop
 // per level, some 250 levels an iteration on a few thousand rows. In krylov.cu a
 // hop is a chain of trips to L1 or L2: the row number, its pointers, its factor
 // values, the neighbours' results, a block barrier or a poll of a value another
-// block stores. Here a block owns a contiguous range of rows (as few blocks as
-// shared memory allows: a hop inside a block is several times shorter than one
-// between blocks), keeps their factor rows, level lists and the swept vector in
-// shared memory, and a hop inside it is: shared-memory reads of the neighbours,
-// the row's operations, a block barrier, with the next level's row already in
-// registers. A value of another block is read from an exchange word
-// (exchange.cuh) that the other block writes when it has the value. Rows are
+// block stores (0.9 us in one block, 2.6 us between blocks). Here a block owns a
+// contiguous range of rows (as few blocks as shared memory allows: a hop inside
+// a block is several times shorter than one between blocks) and keeps their
+// factor rows, level lists and the swept vector in shared memory. A hop inside
+// it is straight-line code: the neighbours' values from shared memory, the row's
+// operations, a barrier of the warps that the widest level needs, with the next
+// level's row already in registers. The values of other blocks (rows within a
+// bandwidth of the range) are brought into shared memory by warps of their own,
+// which poll the exchange words (exchange.cuh) that those blocks write. Rows are
 // taken in level order on every block, so the least unfinished row can always
-// proceed: the blocks are co-resident and a sweep ends. The sums take the
-// layout-independent tree of exchange.cuh.
+// proceed: the blocks are co-resident and a sweep ends.
+//
+// The dot products keep krylov.cu's order for the grid it would have launched:
+// the rows' products go to global memory and are added by the threads that
+// stand for that grid's (grid_sum).
+//
+// Measured on a B200, one PCG iteration (krylov.cu -> here): IC(0) on the 64 x 64
+// cavity (254 levels, 2 blocks) 240 -> 92 us, on 32^3 cells (15 blocks) 600 ->
+// 130 us, ILU(0) on a 65,536-cell channel (RCM order, 29 blocks) 660 -> 290 us. A
+// level costs about 0.3 us with one warp (the FP64 chain of the row: a product and
+// a subtraction an entry, four operations of the quotient), 0.9 us with a thousand
+// rows. 1024 threads (64 registers) were 17 % slower on the cavity and equal on the
+// channel.
 
 #include <algorithm>
 
@@ -26,54 +38,75 @@ namespace mgpu {
 namespace {
 
 constexpr int kSweepThreads = 512;
+constexpr int kPollWarps = 4;  // at least; the warps that no level needs poll too
 
-// A block's rows: sizes, and byte offsets into its shared memory. WO: most
-// off-diagonal entries of a row.
-template <int WO>
+// Marks a value that has not arrived: a signalling NaN, which arithmetic never yields.
+constexpr unsigned long long kPending = 0x7FF0DEAD0BADF00Dull;
+
+// A block's rows: sizes, and byte offsets into its shared memory. W: most
+// entries of a row on one side of the diagonal. A side's arrays are in its level
+// order, each row's entries in the order they apply and padded with (0, the
+// zero), so that a row is read and applied without a branch.
+template <int W>
 struct Sweep {
-  int n, R, start, end, nsc;
-  int wb, bw;        // first row of the column window; largest |column - row|
+  static constexpr int CW = W <= 4 ? 4 : 8;  // places a row
+  int n, R, start, end;
+  int bw;            // largest |column - row|
   int kind;          // 0 ILU(0), 2 IC(0)
-  int cp, cps;       // chunk sums
-  unsigned rseq;     // sums so far
-  double* sums;      // super-chunk sums (2 halves x 2 sums x nsc)
+  double* prod;      // per-row products of the sums (2 halves x 2 sums), see products()
+  double* part;      // krylov.cu's per-block partial sums (2 halves x 2 sums x vgrid)
+  int vgrid;         // krylov.cu's grid: one block of 512 threads, or vgrid of 256
+  unsigned sums;     // sums so far
   unsigned aseq;     // applications so far
   u64 *fwd, *bwd;    // exchange words (pairs) of the forward and backward results
-  int w;             // double[R]: the swept vector
-  int fd;            // double[R]: factor diagonal
-  int fo;            // double[WO][R]: factor off-diagonals of a row, lower entries first, columns ascending
-                     // (IC(0): the upper entries from the transposed factor)
-  int ix;            // unsigned short[WO][R]: their columns, from wb
-  int meta;          // unsigned short[R]: lower entries | upper entries << 4
-  int olo, oup;      // unsigned short[R]: rows in lower / upper level order
-  int plo, pup;      // unsigned short[R + 1]: first of each local level
-  int nlo, nup;      // local levels (those with a row of this block)
+  int w;             // double: the swept vector [0, R), a zero at R, the other blocks' values at [-bw, 0)
+  int fd, fy;        // double[R]: factor diagonal and its reciprocal, by row
+  struct Side {
+    int f;           // double[W][R]: factor entries (IC(0)'s upper side: of the transposed factor)
+    int c;           // unsigned short[R][CW]: where their values are, from the first of the other blocks' values
+    int l;           // unsigned short[R]: row; kPublish: another block may need its value
+    int p;           // unsigned short[R + 1]: first of each local level
+    int nlev;        // local levels (those with a row of this block)
+  } lo, up;
+  int warps;         // warps that the widest of them needs
 };
+constexpr unsigned kPublish = 0x8000u;
 
-constexpr int sweep_row_bytes(int WO) { return 16 + 10 * WO + 2 * 5; }
-inline int sweep_smem(int WO, int R, int cps) { return sweep_row_bytes(WO) * R + 16 + 16 * cps; }
+constexpr int sweep_row_bytes(int W) { return 24 + 2 * (8 * W + 2 * (W <= 4 ? 4 : 8) + 4); }
+inline long sweep_smem(int W, int R, int bw) { return (long)sweep_row_bytes(W) * R + 8l * bw + 64; }
 
-template <int WO>
-__device__ __forceinline__ void sweep_views(Sweep<WO>& S, int R, int cps) {
+template <int W>
+__device__ __forceinline__ void sweep_views(Sweep<W>& S, int R, int bw) {
   S.R = R;
-  S.cps = cps;
-  S.cp = 0;
-  S.w = 16 * cps;
-  S.fd = S.w + 8 * R;
-  S.fo = S.fd + 8 * R;
-  S.ix = S.fo + 8 * WO * R;
-  S.meta = S.ix + 2 * WO * R;
-  S.olo = S.meta + 2 * R;
-  S.oup = S.olo + 2 * R;
-  S.plo = S.oup + 2 * R;
-  S.pup = S.plo + 2 * (R + 1);
+  S.w = 8 * bw;
+  S.fd = S.w + 8 * (R + 1);
+  S.fy = S.fd + 8 * R;
+  int at = (S.fy + 8 * R + 15) & ~15;
+  auto side = [&](typename Sweep<W>::Side& d) {
+    d.c = at;
+    d.f = d.c + 2 * Sweep<W>::CW * R;
+    at = d.f + 8 * W * R;
+  };
+  side(S.lo);
+  side(S.up);
+  S.lo.l = at;
+  S.up.l = S.lo.l + 2 * R;
+  S.lo.p = S.up.l + 2 * R;
+  S.up.p = S.lo.p + 2 * (R + 1);
+}
+
+// the products of the next sum (n; those of a second one n further on): z and w,
+// or the space after the exchange words
+template <int W>
+__device__ __forceinline__ double* products(const Sweep<W>& S) {
+  return S.prod + (S.sums & 1u) * 6l * S.n;
 }
 
 // The block's rows of a level order (ptr, rows: the system's, rows ascending in
 // a level) as local lists; returns the number of local levels. scratch: int[2 * R]
 // in shared memory.
 __device__ __forceinline__ int local_levels(const int* __restrict__ ptr, const int* __restrict__ rows, int nlev,
-                                            int start, int end, int out, int lptr, int scratch) {
+                                            int start, int end, int out, int lptr, int scratch, int& widest) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   __shared__ int s_cnt[32], s_lev[32], s_base[2];
   if (tid == 0) s_base[0] = s_base[1] = 0;
@@ -137,167 +170,245 @@ __device__ __forceinline__ int local_levels(const int* __restrict__ ptr, const i
     const int to = smem_at<unsigned short>(lptr, k);
     for (int j = lane; j < cnt; j += 32) smem_at<unsigned short>(out, to + j) = (unsigned short)(rows[lb + j] - start);
   }
+  int most = 0;
+  for (int k = lane; k < nl; k += 32) most = max(most, smem_at<int>(scratch, 2 * k + 1));
+  widest = max(widest, __reduce_max_sync(0xffffffffu, most));
   __syncthreads();
   return nl;
 }
 
+// A side's rows in its level order: entries, places, and the rows that other
+// blocks may need (those within a bandwidth of the range's end or start).
+template <int W, bool LOWER>
+__device__ __forceinline__ void side_rows(const KrylovArgs& a, const Sweep<W>& S) {
+  const typename Sweep<W>::Side& d = LOWER ? S.lo : S.up;
+  const int rows = S.end - S.start;
+  for (int idx = threadIdx.x; idx < rows; idx += blockDim.x) {
+    const int l = smem_at<unsigned short>(d.l, idx), i = S.start + l;
+    const int di = a.diag[i], k0 = LOWER ? a.row_ptr[i] : di + 1, k1 = LOWER ? di : a.row_ptr[i + 1];
+#pragma unroll
+    for (int t = 0; t < W; ++t) {
+      const bool in = k0 + t < k1;
+      // IC(0)'s backward sweep applies the entries in descending column order
+      const int k = !LOWER && S.kind == 2 ? k1 - 1 - t : k0 + t;
+      int place = S.bw + S.R;
+      double f = 0.0;
+      if (in) {
+        f = a.fval[!LOWER && S.kind == 2 ? a.lt_pos[k] : k];
+        const int c = a.col[k] - S.start;
+        // the rows after the range share the places of those before it
+        place = (unsigned)c < (unsigned)S.R ? S.bw + c : LOWER ? S.bw + c : c - S.R;
+      }
+      smem_at<double>(d.f, t * S.R + idx) = f;
+      smem_at<unsigned short>(d.c, idx * Sweep<W>::CW + t) = (unsigned short)place;
+    }
+    const bool out = LOWER ? l + S.bw >= rows && S.end < S.n : l < S.bw && S.start > 0;
+    if (out) smem_at<unsigned short>(d.l, idx) = (unsigned short)(l | kPublish);
+  }
+}
+
 // The block's part of the system in shared memory, its words cleared; the
 // barrier puts every block's clears (and zeroed x) before what follows.
-template <int WO, int K>
-__device__ __forceinline__ bool sweep_prologue(const KrylovArgs& a, VGrid& g, Sweep<WO>& S) {
-  const int T = blockDim.x, tid = threadIdx.x;
-  S.wb = max(0, S.start - S.bw);
-  S.nlo = local_levels(a.lo_ptr, a.lo_rows, a.nlev_lo, S.start, S.end, S.olo, S.plo, S.fo);
-  S.nup = local_levels(a.up_ptr, a.up_rows, a.nlev_up, S.start, S.end, S.oup, S.pup, S.fo);
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int l = k * T + tid, i = S.start + l;
-    if (i >= S.end) continue;
-    const int rb = a.row_ptr[i], re = a.row_ptr[i + 1], di = a.diag[i];
-    const int nl = di - rb;
-#pragma unroll
-    for (int t = 0; t < WO; ++t)
-      if (rb + t + (t >= nl) < re) {
-        const int e = rb + t + (t >= nl);  // the diagonal is skipped
-        smem_at<double>(S.fo, t * S.R + l) = a.fval[S.kind == 2 && t >= nl ? a.lt_pos[e] : e];
-        smem_at<unsigned short>(S.ix, t * S.R + l) = (unsigned short)(a.col[e] - S.wb);
-      }
-    smem_at<double>(S.fd, l) = a.fval[di];
-    smem_at<unsigned short>(S.meta, l) = (unsigned short)(nl | (re - di - 1) << 4);
+template <int W>
+__device__ __forceinline__ bool sweep_prologue(const KrylovArgs& a, VGrid& g, Sweep<W>& S) {
+  int widest = 0;
+  S.lo.nlev = local_levels(a.lo_ptr, a.lo_rows, a.nlev_lo, S.start, S.end, S.lo.l, S.lo.p, S.lo.f, widest);
+  S.up.nlev = local_levels(a.up_ptr, a.up_rows, a.nlev_up, S.start, S.end, S.up.l, S.up.p, S.lo.f, widest);
+  S.warps = min((widest + 31) / 32, (int)(blockDim.x >> 5) - kPollWarps);
+  for (int i = S.start + threadIdx.x; i < S.end; i += blockDim.x) {
+    const double d = a.fval[a.diag[i]];
+    smem_at<double>(S.fd, i - S.start) = d;
+    smem_at<double>(S.fy, i - S.start) = 1.0 / d;
     S.fwd[2l * i] = S.fwd[2l * i + 1] = 0ull;
     S.bwd[2l * i] = S.bwd[2l * i + 1] = 0ull;
     if (a.zero_x) a.x[i] = 0.0;
   }
+  side_rows<W, true>(a, S);
+  side_rows<W, false>(a, S);
+  if (threadIdx.x == 0) smem_at<double>(S.w, S.R) = 0.0;
   return vg_sync(g, a.st);
 }
 
+// s / d from y = 1 / d rounded to nearest: two corrections of the quotient by
+// its exact remainder (P. Markstein, Computation of elementary functions on the
+// IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990: with y correctly
+// rounded and q within an ulp, q + (s - q d) y rounds to the quotient). Only
+// these four operations wait for s. Outside the exponents where no intermediate
+// can over- or underflow, the division itself.
+__device__ __forceinline__ double quotient(double s, double d, double y) {
+  const int es = (__double2hiint(s) >> 20) & 0x7ff, ed = (__double2hiint(d) >> 20) & 0x7ff;
+  double q = s * y;
+  q = fma(fma(-d, q, s), y, q);
+  q = fma(fma(-d, q, s), y, q);
+  const bool plain = (unsigned)(es - 512) < 1024u && (unsigned)(ed - 800) < 448u;
+  return plain ? q : s / d;
+}
+
 // A row of the next level, read ahead of the barrier before it.
-template <int WO>
+template <int W>
 struct Fetched {
-  int l;  // local row (-1: none)
-  int m;  // entries to apply
-  double f[WO];
-  int c[WO];  // their columns, from the block's first row
-  double fd;
+  unsigned l;    // its number, with kPublish
+  double f[W];
+  unsigned c[W];  // byte offsets of the values
 };
 
-template <int WO, bool FWD>
-__device__ __forceinline__ void fetch_row(const Sweep<WO>& S, int idx, int e, Fetched<WO>& r) {
-  r.l = -1;
-  if (idx >= e) return;
-  const int l = smem_at<unsigned short>(FWD ? S.olo : S.oup, idx);
-  const unsigned meta = smem_at<unsigned short>(S.meta, l);
-  const int nl = meta & 15u, nu = meta >> 4, off = S.wb - S.start;
-  r.l = l;
-  r.m = FWD ? nl : nu;
-  r.fd = smem_at<double>(S.fd, l);
+template <int W>
+__device__ __forceinline__ void fetch_row(const Sweep<W>& S, const typename Sweep<W>::Side& d, int idx,
+                                          Fetched<W>& r) {
+  r.l = smem_at<unsigned short>(d.l, idx);
+  unsigned pk[Sweep<W>::CW / 2];
+  if constexpr (W <= 4) {
+    const uint2 c = smem_at<uint2>(d.c, idx);
+    pk[0] = c.x;
+    pk[1] = c.y;
+  } else {
+    const uint4 c = smem_at<uint4>(d.c, idx);
+    pk[0] = c.x;
+    pk[1] = c.y;
+    pk[2] = c.z;
+    pk[3] = c.w;
+  }
 #pragma unroll
-  for (int t = 0; t < WO; ++t)
-    if (t < r.m) {
-      // IC(0)'s backward sweep applies the entries in descending column order
-      const int p = FWD ? t : (S.kind == 2 ? nl + nu - 1 - t : nl + t);
-      r.f[t] = smem_at<double>(S.fo, p * S.R + l);
-      r.c[t] = (int)smem_at<unsigned short>(S.ix, p * S.R + l) + off;
-    }
+  for (int t = 0; t < W; ++t) {
+    r.f[t] = smem_at<double>(d.f, t * S.R + idx);
+    r.c[t] = t & 1 ? pk[t / 2] >> 16 : pk[t / 2] & 0xffffu;
+  }
 }
 
-template <int WO, bool FWD>
-__device__ __forceinline__ bool sweep_row(const Sweep<WO>& S, const Fetched<WO>& r, DevStatus* st) {
-  const u64* words = FWD ? S.fwd : S.bwd;
-  double v[WO];
-  bool ok = true;
+__device__ __forceinline__ double ld_value(unsigned place) {
+  double v;
+  const unsigned at = (unsigned)__cvta_generic_to_shared(block_smem) + 8u * place;
+  asm volatile("ld.relaxed.cta.shared.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_value(unsigned place, double v) {
+  const unsigned at = (unsigned)__cvta_generic_to_shared(block_smem) + 8u * place;
+  asm volatile("st.relaxed.cta.shared.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+__device__ __forceinline__ bool pending(double v) { return (u64)__double_as_longlong(v) == kPending; }
+
+template <int W, bool FWD>
+__device__ __forceinline__ bool sweep_row(const Sweep<W>& S, const Fetched<W>& r, DevStatus* st) {
+  const unsigned l = r.l & (kPublish - 1u);
+  double v[W], d = 1.0, y = 1.0;
+  bool ok = true, wait = false;
 #pragma unroll
-  for (int t = 0; t < WO; ++t)
-    if (t < r.m) {
-      if ((unsigned)r.c[t] < (unsigned)S.R) {
-        v[t] = smem_at<double>(S.w, r.c[t]);
-      } else {
-        const u64* p = words + 2l * (S.start + r.c[t]);
-        u64 lo, hi;
-        ld_pair(p, lo, hi);
-        unsigned spins = 0;
-        while (((unsigned)(lo >> 32) != S.aseq || (unsigned)(hi >> 32) != S.aseq) && ok) {
-          ok = keep_polling(spins, st);
-          ld_pair(p, lo, hi);
-        }
-        v[t] = __longlong_as_double((long long)((hi << 32) | (lo & 0xffffffffull)));
+  for (int t = 0; t < W; ++t) v[t] = ld_value(r.c[t]);
+  double s = ld_value(S.bw + l);
+  const bool divide = !FWD || S.kind == 2;
+  if (divide) {
+    d = smem_at<double>(S.fd, l);
+    y = smem_at<double>(S.fy, l);
+  }
+#pragma unroll
+  for (int t = 0; t < W; ++t) wait = wait || pending(v[t]);
+  if (wait) {
+    unsigned spins = 0;
+#pragma unroll
+    for (int t = 0; t < W; ++t)
+      while (pending(v[t]) && ok) {
+        ok = keep_polling(spins, st);
+        v[t] = ld_value(r.c[t]);
+      }
+  }
+#pragma unroll
+  for (int t = 0; t < W; ++t) s = s - r.f[t] * v[t];
+  if (divide) s = quotient(s, d, y);
+  st_value(S.bw + l, s);
+  if (r.l & kPublish) st_pair((FWD ? S.fwd : S.bwd) + 2l * (S.start + (int)l), s, S.aseq);
+  return ok;
+}
+
+// The levels in order, by the first S.warps warps; bar.sync 1 is theirs.
+template <int W, bool FWD>
+__device__ __forceinline__ bool sweep_levels(const Sweep<W>& S, DevStatus* st) {
+  const typename Sweep<W>::Side& d = FWD ? S.lo : S.up;
+  const int tid = threadIdx.x, T = 32 * S.warps, nlev = d.nlev, rows = S.end - S.start;
+  bool ok = true;
+  Fetched<W> r;
+  int b = tid, e = smem_at<unsigned short>(d.p, 1), e1 = smem_at<unsigned short>(d.p, min(2, nlev));
+  fetch_row<W>(S, d, min(b, rows - 1), r);
+  for (int lev = 0; lev < nlev; ++lev) {
+    if (b < e) ok = sweep_row<W, FWD>(S, r, st) && ok;
+    for (int idx = b + T; idx < e; idx += T) {
+      fetch_row<W>(S, d, idx, r);
+      ok = sweep_row<W, FWD>(S, r, st) && ok;
+    }
+    b = e + tid;
+    e = e1;
+    e1 = smem_at<unsigned short>(d.p, min(lev + 3, nlev));
+    fetch_row<W>(S, d, min(b, rows - 1), r);
+    asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory");
+  }
+  return ok;
+}
+
+// The other warps: the values of the rows before the range (forward) or after it
+// (backward) as their blocks write them, each thread taking its rows in turn
+// without waiting for any one of them.
+template <int W, bool FWD>
+__device__ __forceinline__ bool sweep_poll(const Sweep<W>& S, DevStatus* st) {
+  const int P = (int)blockDim.x - 32 * S.warps, tid = (int)threadIdx.x - 32 * S.warps;
+  const u64* words = FWD ? S.fwd : S.bwd;
+  const int first = FWD ? S.start - S.bw : S.end;  // row of place -bw
+  unsigned left = 0u;
+  for (int k = 0, j = tid; j < S.bw; j += P, ++k)
+    if (first + j >= 0 && first + j < S.n) left |= 1u << k;
+  unsigned spins = 0;
+  while (left) {
+    for (unsigned m = left; m; m &= m - 1u) {
+      const int k = __ffs(m) - 1, j = tid + k * P;
+      u64 lo, hi;
+      ld_pair(words + 2l * (first + j), lo, hi);
+      if ((unsigned)(lo >> 32) == S.aseq && (unsigned)(hi >> 32) == S.aseq) {
+        st_value(j, __longlong_as_double((long long)((hi << 32) | (lo & 0xffffffffull))));
+        left &= ~(1u << k);
       }
     }
-  double s = smem_at<double>(S.w, r.l);
-#pragma unroll
-  for (int t = 0; t < WO; ++t)
-    if (t < r.m) s = s - r.f[t] * v[t];
-  if (!FWD || S.kind == 2) s = s / r.fd;
-  smem_at<double>(S.w, r.l) = s;
-  // rows within a bandwidth of the range's end (forward) or start (backward)
-  // may be another block's neighbours
-  const bool out = FWD ? r.l + S.bw >= S.end - S.start && S.end < S.n : r.l < S.bw && S.start > 0;
-  if (out) st_pair(const_cast<u64*>(words) + 2l * (S.start + r.l), s, S.aseq);
-  return ok;
+    if (left && !keep_polling(spins, st)) return false;
+  }
+  return true;
 }
 
-template <int WO, bool FWD>
-__device__ __forceinline__ bool sweep_half(const Sweep<WO>& S, DevStatus* st) {
-  const int tid = threadIdx.x, T = blockDim.x;
-  const int nlev = FWD ? S.nlo : S.nup, ptr = FWD ? S.plo : S.pup;
-  bool ok = true;
-  Fetched<WO> r;
-  int e = smem_at<unsigned short>(ptr, 1);
-  fetch_row<WO, FWD>(S, smem_at<unsigned short>(ptr, 0) + tid, e, r);
-  for (int lev = 0; lev < nlev; ++lev) {
-    if (r.l >= 0) ok = sweep_row<WO, FWD>(S, r, st) && ok;
-    for (int idx = smem_at<unsigned short>(ptr, lev) + T + tid; idx < e; idx += T) {
-      fetch_row<WO, FWD>(S, idx, e, r);
-      ok = sweep_row<WO, FWD>(S, r, st) && ok;
-    }
-    r.l = -1;
-    if (lev + 1 < nlev) {
-      const int b = e;
-      e = smem_at<unsigned short>(ptr, lev + 2);
-      fetch_row<WO, FWD>(S, b + tid, e, r);
-    }
-    __syncthreads();
-  }
-  return ok;
-}
-
-// z = M^-1 src for the block's rows (z[k] of this thread's row in tile k). The
-// words of an application are written again only after a sum over all blocks,
-// which each block joins when it has read all it needs.
-template <int WO, int K>
-__device__ __forceinline__ bool sweep_apply(Sweep<WO>& S, const double (&src)[K], double (&z)[K], DevStatus* st) {
-  const int T = blockDim.x, tid = threadIdx.x;
-  ++S.aseq;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int l = k * T + tid;
-    if (S.start + l < S.end) smem_at<double>(S.w, l) = src[k];
-  }
+template <int W, bool FWD>
+__device__ __forceinline__ bool sweep_half(const Sweep<W>& S, DevStatus* st) {
+  for (int j = threadIdx.x; j < S.bw; j += blockDim.x)
+    st_value(j, __longlong_as_double((long long)kPending));
   __syncthreads();
-  bool ok = sweep_half<WO, true>(S, st);
-  ok = sweep_half<WO, false>(S, st) && ok;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int l = k * T + tid;
-    z[k] = S.start + l < S.end ? smem_at<double>(S.w, l) : 0.0;
-  }
+  const bool ok = (int)threadIdx.x < 32 * S.warps ? sweep_levels<W, FWD>(S, st) : sweep_poll<W, FWD>(S, st);
   return __syncthreads_and(ok) != 0;
 }
 
-// y_i = A_i . x in csr_matvec order
+// dst = M^-1 src on the block's rows. The words of an application are written
+// again only after a sum or barrier over all blocks, which each block joins when
+// it has read all it needs.
+template <int W>
+__device__ __forceinline__ bool sweep_apply(Sweep<W>& S, const double* src, double* dst, DevStatus* st) {
+  const int n = S.end - S.start;
+  ++S.aseq;
+  for (int l = threadIdx.x; l < n; l += blockDim.x) smem_at<double>(S.w, l) = src[S.start + l];
+  if (!sweep_half<W, true>(S, st) || !sweep_half<W, false>(S, st)) return false;
+  for (int l = threadIdx.x; l < n; l += blockDim.x) dst[S.start + l] = smem_at<double>(S.w, l);
+  return true;
+}
+
+// y_i = A_i . x in csr_matvec order, the row's first 8 loads issued together
 __device__ __forceinline__ double row_product(const KrylovArgs& a, const double* x, int i) {
   const int b = a.row_ptr[i], e = a.row_ptr[i + 1];
   double v[8], xv[8];
 #pragma unroll
-  for (int t = 0; t < 8; ++t)
+  for (int t = 0; t < 8; ++t) {
+    v[t] = xv[t] = 0.0;
     if (b + t < e) {
       v[t] = a.aval[b + t];
       xv[t] = ldv(&x[a.col[b + t]]);
     }
+  }
   double y = 0.0;
 #pragma unroll
   for (int t = 0; t < 8; ++t)
     if (b + t < e) y = y + v[t] * xv[t];
+  for (int k = b + 8; k < e; ++k) y = y + a.aval[k] * ldv(&x[a.col[k]]);
   return y;
 }
 
@@ -316,69 +427,114 @@ __device__ __forceinline__ void sweep_result(const KrylovArgs& a, int it, double
   }
 }
 
-template <int WO, int K>
-__device__ __forceinline__ void sweep_begin(const KrylovArgs& a, const VGrid& g, Sweep<WO>& S, int R, int bw) {
+// The sums of the products (every block has written its
+// rows') in the order of krylov.cu's vg_sum: on one block of 512 threads each
+// adds its rows in steps of 512, then butterflies over the warps and over the 16
+// warp sums; on vgrid blocks of 256, each thread its rows in steps of the grid,
+// butterflies within its block, and the blocks' partial sums in a fixed order of
+// 256 threads. Every block of this launch computes all (the partials: its share).
+template <int NQ, int W>
+__device__ __forceinline__ bool grid_sum(Sweep<W>& S, VGrid& g, DevStatus* st, double (&out)[NQ]) {
+  __shared__ double s_warp[2][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned half = S.sums & 1u;
+  const double* c = products(S);
+  ++S.sums;
+  if (!vg_sync(g, st)) return false;
+  if (S.vgrid == 1) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      double v = 0.0;
+#pragma unroll 8
+      for (int i = tid; i < S.n; i += 512) v = v + ldv(&c[(long)q * S.n + i]);
+      v = warp_sum(v);
+      if (lane == 0) s_warp[q][warp] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) out[q] = warp_sum(lane < 16 ? s_warp[q][lane] : 0.0);
+    __syncthreads();
+    return true;
+  }
+  const int vb = S.vgrid, step = 256 * vb;
+  double* part = S.part + half * 2l * vb;
+  for (int b0 = 2 * g.rank; b0 < vb; b0 += 2 * g.nb) {
+    const int b = b0 + (tid >> 8);  // two of its blocks side by side
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      double v = 0.0;
+      if (b < vb)
+        for (int i = 256 * b + (tid & 255); i < S.n; i += step) v = v + ldv(&c[(long)q * S.n + i]);
+      v = warp_sum(v);
+      if (lane == 0) s_warp[q][warp] = v;
+    }
+    __syncthreads();
+    if ((warp & 7) == 0 && b < vb) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const double v = warp_sum(lane < 8 ? s_warp[q][warp + lane] : 0.0);
+        if (lane == 0) part[(long)q * vb + b] = v;
+      }
+    }
+    __syncthreads();
+  }
+  if (!vg_sync(g, st)) return false;
+  if (warp < 8) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const double* p = part + (long)q * vb;
+      double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
+      if (tid < vb) t0 = ldv(&p[tid]);
+      if (tid + 256 < vb) t1 = ldv(&p[tid + 256]);
+      if (tid + 512 < vb) t2 = ldv(&p[tid + 512]);
+      if (tid + 768 < vb) t3 = ldv(&p[tid + 768]);
+      double v = ((t0 + t1) + t2) + t3;
+      for (int j = tid + 1024; j < vb; j += 256) v = v + ldv(&p[j]);
+      v = warp_sum(v);
+      if (lane == 0) s_warp[q][warp] = v;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) out[q] = warp_sum(lane < 8 ? s_warp[q][lane] : 0.0);
+  __syncthreads();
+  return true;
+}
+
+template <int W>
+__device__ __forceinline__ void sweep_begin(const KrylovArgs& a, const VGrid& g, Sweep<W>& S, int R, int vgrid) {
   S.n = a.n;
-  S.bw = bw;
+  S.bw = a.bw;
   S.kind = a.precond;
   S.start = g.rank * R;
   S.end = min(a.n, S.start + R);
-  S.nsc = (a.n + kSuperRows - 1) / kSuperRows;
-  S.rseq = S.aseq = 0u;
-  S.sums = a.z;
-  sweep_views<WO>(S, R, K * (blockDim.x / 32));
+  S.aseq = S.sums = 0u;
+  double* more = a.w + a.n;  // 6 n more than krylov.cu's work vectors
+  S.fwd = reinterpret_cast<u64*>(more);
+  S.bwd = reinterpret_cast<u64*>(more + 2l * a.n);
+  S.prod = a.z;
+  S.part = a.partials;
+  S.vgrid = vgrid;
+  sweep_views<W>(S, R, a.bw);
 }
 
-// the rows of this thread: f(tile k, row i)
-#define MGPU_OWN_ROWS(k, i)                                        \
-  _Pragma("unroll") for (int k = 0; k < K; ++k)                    \
-    if (const int i = S.start + k * (int)blockDim.x + (int)threadIdx.x; i < S.end)
-
-// sum over all rows of the per-row values c0[k] (c1[k]) into out
-template <int K, typename State>
-__device__ __forceinline__ bool sum1(State& S, VGrid& g, DevStatus* st, const double (&c0)[K], double& out) {
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const double c[1] = {c0[k]};
-    resident_put<1>(S.cp, S.cps, k, c);
-  }
-  double t[1];
-  if (!resident_total<1>(S, g, st, t)) return false;
-  out = t[0];
-  return true;
-}
-template <int K, typename State>
-__device__ __forceinline__ bool sum2(State& S, VGrid& g, DevStatus* st, const double (&c0)[K], const double (&c1)[K],
-                                     double (&out)[2]) {
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const double c[2] = {c0[k], c1[k]};
-    resident_put<2>(S.cp, S.cps, k, c);
-  }
-  return resident_total<2>(S, g, st, out);
-}
+#define MGPU_OWN_ROWS(i) for (int i = S.start + (int)threadIdx.x; i < S.end; i += (int)blockDim.x)
 
 // k_pcg (krylov.cu) with ILU(0) or IC(0)
-template <int WO, int K>
-__global__ void __launch_bounds__(kSweepThreads, 1) k_pcg_sweep(KrylovArgs a, int R, int bw) {
+template <int W>
+__global__ void __launch_bounds__(kSweepThreads, 1) k_pcg_sweep(KrylovArgs a, int R, int vgrid) {
   if (a.st->abort) return;
   VGrid g = whole_grid(a.bar, a.partials, true);
-  Sweep<WO> S;
-  sweep_begin<WO, K>(a, g, S, R, bw);
-  S.fwd = reinterpret_cast<u64*>(a.s);   // s, t
-  S.bwd = reinterpret_cast<u64*>(a.ph);  // ph, sh
-  double* x = a.x;
-  double* p = a.p;
-  double r[K], z[K], q[K], pk[K], c[K];
-  if (!sweep_prologue<WO, K>(a, g, S)) return;
-#pragma unroll
-  for (int k = 0; k < K; ++k) r[k] = z[k] = q[k] = pk[k] = c[k] = 0.0;
-  MGPU_OWN_ROWS(k, i) c[k] = a.b[i] * a.b[i];
-  double bb;
-  if (!sum1<K>(S, g, a.st, c, bb)) return;
-  const double bnrm = sqrt(bb);
+  Sweep<W> S;
+  sweep_begin<W>(a, g, S, R, vgrid);
+  double *x = a.x, *r = a.r, *p = a.p, *q = a.v, *z = a.r0;
+  if (!sweep_prologue<W>(a, g, S)) return;
+  double t[1];
+  MGPU_OWN_ROWS(i) products(S)[i] = a.b[i] * a.b[i];
+  if (!grid_sum<1>(S, g, a.st, t)) return;
+  const double bnrm = sqrt(t[0]);
   if (bnrm == 0.0) {
-    MGPU_OWN_ROWS(k, i) x[i] = 0.0;
+    MGPU_OWN_ROWS(i) x[i] = 0.0;
     sweep_result(a, 0, 0.0, 0);
     return;
   }
@@ -386,92 +542,82 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_pcg_sweep(KrylovArgs a, in
     sweep_result(a, 0, 0.0, *a.ferr + 10);
     return;
   }
-  MGPU_OWN_ROWS(k, i) {
-    r[k] = a.b[i] - row_product(a, x, i);
-    c[k] = r[k] * r[k];
+  MGPU_OWN_ROWS(i) {
+    const double ri = a.b[i] - row_product(a, x, i);
+    r[i] = ri;
+    products(S)[i] = ri * ri;
   }
-  double rr;
-  if (!sum1<K>(S, g, a.st, c, rr)) return;
-  double res = sqrt(rr) / bnrm;
+  if (!grid_sum<1>(S, g, a.st, t)) return;
+  double res = sqrt(t[0]) / bnrm;
   if (res <= a.tol) {
     sweep_result(a, 0, res, 0);
     return;
   }
-  double rz;
-  if (!sweep_apply<WO, K>(S, r, z, a.st)) return;
-#pragma unroll
-  for (int k = 0; k < K; ++k) c[k] = r[k] * z[k];
-  MGPU_OWN_ROWS(k, i) {
-    pk[k] = z[k];
-    p[i] = pk[k];
+  if (!sweep_apply(S, r, z, a.st)) return;
+  MGPU_OWN_ROWS(i) {
+    const double zi = z[i];
+    p[i] = zi;
+    products(S)[i] = r[i] * zi;
   }
-  if (!sum1<K>(S, g, a.st, c, rz)) return;  // its barrier shows every block's p
+  if (!grid_sum<1>(S, g, a.st, t)) return;  // its barrier shows every block's p
+  double rz = t[0];
   int ierr = 0, it;
   for (it = 1; it <= a.maxit; ++it) {
-    MGPU_OWN_ROWS(k, i) {
-      q[k] = row_product(a, p, i);
-      c[k] = pk[k] * q[k];
+    MGPU_OWN_ROWS(i) {
+      const double qi = row_product(a, p, i);
+      q[i] = qi;
+      products(S)[i] = p[i] * qi;
     }
-    double pap;
-    if (!sum1<K>(S, g, a.st, c, pap)) return;
+    if (!grid_sum<1>(S, g, a.st, t)) return;
+    const double pap = t[0];
     if (fabs(pap) < DTINY) {
       ierr = 2;
       break;
     }
     const double alpha = rz / pap;
-    MGPU_OWN_ROWS(k, i) {
-      x[i] = x[i] + alpha * pk[k];
-      r[k] = r[k] - alpha * q[k];
-      c[k] = r[k] * r[k];
+    MGPU_OWN_ROWS(i) {
+      x[i] = x[i] + alpha * p[i];
+      const double ri = r[i] - alpha * q[i];
+      r[i] = ri;
+      products(S)[i] = ri * ri;
     }
-    if (!sum1<K>(S, g, a.st, c, rr)) return;
-    res = sqrt(rr) / bnrm;
+    if (!grid_sum<1>(S, g, a.st, t)) return;
+    res = sqrt(t[0]) / bnrm;
     if (res <= a.tol) {
       sweep_result(a, it, res, 0);
       return;
     }
-    double rz_new;
-    if (!sweep_apply<WO, K>(S, r, z, a.st)) return;
-#pragma unroll
-    for (int k = 0; k < K; ++k) c[k] = r[k] * z[k];
-    if (!sum1<K>(S, g, a.st, c, rz_new)) return;
+    if (!sweep_apply(S, r, z, a.st)) return;
+    MGPU_OWN_ROWS(i) products(S)[i] = r[i] * z[i];
+    if (!grid_sum<1>(S, g, a.st, t)) return;
     if (fabs(rz) < DTINY) {
       ierr = 2;
       break;
     }
-    const double beta = rz_new / rz;
-    MGPU_OWN_ROWS(k, i) {
-      pk[k] = z[k] + beta * pk[k];
-      p[i] = pk[k];
-    }
+    const double beta = t[0] / rz;
+    MGPU_OWN_ROWS(i) p[i] = z[i] + beta * p[i];
     if (!vg_sync(g, a.st)) return;
-    rz = rz_new;
+    rz = t[0];
   }
   if (ierr == 0) ierr = 1;
   sweep_result(a, it, res, ierr);
 }
 
 // k_bicgstab (krylov.cu) with ILU(0)
-template <int WO, int K>
-__global__ void __launch_bounds__(kSweepThreads, 1) k_bicgstab_sweep(KrylovArgs a, int R, int bw) {
+template <int W>
+__global__ void __launch_bounds__(kSweepThreads, 1) k_bicgstab_sweep(KrylovArgs a, int R, int vgrid) {
   if (a.st->abort) return;
   VGrid g = whole_grid(a.bar, a.partials, true);
-  Sweep<WO> S;
-  sweep_begin<WO, K>(a, g, S, R, bw);
-  S.fwd = reinterpret_cast<u64*>(a.p);  // p, v
-  S.bwd = reinterpret_cast<u64*>(a.s);  // s, t
-  double* x = a.x;
-  double *r0 = a.r0, *ph = a.ph, *sh = a.sh;
-  double r[K], p[K], v[K], y[K], z[K], t[K], c[K], e[K];
-  if (!sweep_prologue<WO, K>(a, g, S)) return;
-#pragma unroll
-  for (int k = 0; k < K; ++k) r[k] = p[k] = v[k] = y[k] = z[k] = t[k] = c[k] = e[k] = 0.0;
-  MGPU_OWN_ROWS(k, i) c[k] = a.b[i] * a.b[i];
-  double bb;
-  if (!sum1<K>(S, g, a.st, c, bb)) return;
-  const double bnrm = sqrt(bb);
+  Sweep<W> S;
+  sweep_begin<W>(a, g, S, R, vgrid);
+  double *x = a.x, *r = a.r, *r0 = a.r0, *p = a.p, *v = a.v, *s = a.s, *t = a.t, *ph = a.ph, *sh = a.sh;
+  if (!sweep_prologue<W>(a, g, S)) return;
+  double t1[1];
+  MGPU_OWN_ROWS(i) products(S)[i] = a.b[i] * a.b[i];
+  if (!grid_sum<1>(S, g, a.st, t1)) return;
+  const double bnrm = sqrt(t1[0]);
   if (bnrm == 0.0) {
-    MGPU_OWN_ROWS(k, i) x[i] = 0.0;
+    MGPU_OWN_ROWS(i) x[i] = 0.0;
     sweep_result(a, 0, 0.0, 0);
     return;
   }
@@ -479,19 +625,21 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_bicgstab_sweep(KrylovArgs 
     sweep_result(a, 0, 0.0, *a.ferr + 10);
     return;
   }
-  MGPU_OWN_ROWS(k, i) {
-    r[k] = a.b[i] - row_product(a, x, i);
-    r0[i] = r[k];
-    c[k] = r[k] * r[k];
+  MGPU_OWN_ROWS(i) {
+    const double ri = a.b[i] - row_product(a, x, i);
+    r0[i] = ri;
+    r[i] = ri;
+    p[i] = 0.0;
+    v[i] = 0.0;
+    products(S)[i] = ri * ri;
   }
-  double rho_next;
-  if (!sum1<K>(S, g, a.st, c, rho_next)) return;
-  double res = sqrt(rho_next) / bnrm;
+  if (!grid_sum<1>(S, g, a.st, t1)) return;
+  double res = sqrt(t1[0]) / bnrm;
   if (res <= a.tol) {
     sweep_result(a, 0, res, 0);
     return;
   }
-  double rho_old = 1.0, alpha = 1.0, omega = 1.0;
+  double rho_next = t1[0], rho_old = 1.0, alpha = 1.0, omega = 1.0;
   int ierr = 0, it;
   for (it = 1; it <= a.maxit; ++it) {
     const double rho = rho_next;
@@ -500,66 +648,62 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_bicgstab_sweep(KrylovArgs 
       break;
     }
     const double beta = (rho / rho_old) * (alpha / omega);
-#pragma unroll
-    for (int k = 0; k < K; ++k) p[k] = r[k] + beta * (p[k] - omega * v[k]);
-    if (!sweep_apply<WO, K>(S, p, y, a.st)) return;
-    MGPU_OWN_ROWS(k, i) ph[i] = y[k];
+    MGPU_OWN_ROWS(i) p[i] = r[i] + beta * (p[i] - omega * v[i]);
+    if (!sweep_apply(S, p, ph, a.st)) return;
     if (!vg_sync(g, a.st)) return;
-    MGPU_OWN_ROWS(k, i) {
-      v[k] = row_product(a, ph, i);
-      c[k] = r0[i] * v[k];
+    MGPU_OWN_ROWS(i) {
+      const double vi = row_product(a, ph, i);
+      v[i] = vi;
+      products(S)[i] = r0[i] * vi;
     }
-    double d1;
-    if (!sum1<K>(S, g, a.st, c, d1)) return;
-    alpha = rho / d1;
-    // r becomes s
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      r[k] = r[k] - alpha * v[k];
-      c[k] = r[k] * r[k];
+    if (!grid_sum<1>(S, g, a.st, t1)) return;
+    alpha = rho / t1[0];
+    MGPU_OWN_ROWS(i) {
+      const double si = r[i] - alpha * v[i];
+      s[i] = si;
+      products(S)[i] = si * si;
     }
-    double d2;
-    if (!sum1<K>(S, g, a.st, c, d2)) return;
-    const double snrm = sqrt(d2);
+    if (!grid_sum<1>(S, g, a.st, t1)) return;
+    const double snrm = sqrt(t1[0]);
     if (snrm / bnrm <= a.tol) {
-      MGPU_OWN_ROWS(k, i) x[i] = x[i] + alpha * y[k];
+      MGPU_OWN_ROWS(i) x[i] = x[i] + alpha * ph[i];
       sweep_result(a, it, snrm / bnrm, 0);
       return;
     }
-    if (!sweep_apply<WO, K>(S, r, z, a.st)) return;
-    MGPU_OWN_ROWS(k, i) sh[i] = z[k];
+    if (!sweep_apply(S, s, sh, a.st)) return;
     if (!vg_sync(g, a.st)) return;
-    MGPU_OWN_ROWS(k, i) {
-      t[k] = row_product(a, sh, i);
-      c[k] = t[k] * t[k];
-      e[k] = t[k] * r[k];
+    MGPU_OWN_ROWS(i) {
+      const double ti = row_product(a, sh, i);
+      t[i] = ti;
+      products(S)[i] = ti * ti;
+      products(S)[S.n + i] = ti * s[i];
     }
-    double d3[2];
-    if (!sum2<K>(S, g, a.st, c, e, d3)) return;
-    const double tt = d3[0];
+    double t2[2];
+    if (!grid_sum<2>(S, g, a.st, t2)) return;
+    const double tt = t2[0];
     if (tt < DTINY) {
       ierr = 2;
       break;
     }
-    omega = d3[1] / tt;
+    omega = t2[1] / tt;
     if (fabs(omega) < DTINY) {
       ierr = 2;
       break;
     }
-    MGPU_OWN_ROWS(k, i) {
-      x[i] = x[i] + alpha * y[k] + omega * z[k];
-      r[k] = r[k] - omega * t[k];
-      c[k] = r[k] * r[k];
-      e[k] = r[k] * r0[i];
+    MGPU_OWN_ROWS(i) {
+      x[i] = x[i] + alpha * ph[i] + omega * sh[i];
+      const double ri = s[i] - omega * t[i];
+      r[i] = ri;
+      products(S)[i] = ri * ri;
+      products(S)[S.n + i] = ri * r0[i];
     }
-    double d4[2];
-    if (!sum2<K>(S, g, a.st, c, e, d4)) return;
-    res = sqrt(d4[0]) / bnrm;
+    if (!grid_sum<2>(S, g, a.st, t2)) return;
+    res = sqrt(t2[0]) / bnrm;
     if (res <= a.tol) {
       sweep_result(a, it, res, 0);
       return;
     }
-    rho_next = d4[1];
+    rho_next = t2[1];
     rho_old = rho;
   }
   if (ierr == 0) {
@@ -570,45 +714,42 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_bicgstab_sweep(KrylovArgs 
 }
 #undef MGPU_OWN_ROWS
 
-template <int WO>
-const void* sweep_kernel(int K, bool pcg) {
-  switch (K) {
-    case 1: return pcg ? (const void*)k_pcg_sweep<WO, 1> : (const void*)k_bicgstab_sweep<WO, 1>;
-    case 2: return pcg ? (const void*)k_pcg_sweep<WO, 2> : (const void*)k_bicgstab_sweep<WO, 2>;
-    case 4: return pcg ? (const void*)k_pcg_sweep<WO, 4> : (const void*)k_bicgstab_sweep<WO, 4>;
-    default: return pcg ? (const void*)k_pcg_sweep<WO, 6> : (const void*)k_bicgstab_sweep<WO, 6>;
-  }
-}
-
 }  // namespace
 
-// The resident solve of a factored system whose rows have at most 7 entries and
-// fit in the SMs' shared memory, column windows in 16 bits; *taken = false and
-// no launch otherwise.
+template <int W>
+const void* sweep_kernel(bool pcg) {
+  return pcg ? (const void*)k_pcg_sweep<W> : (const void*)k_bicgstab_sweep<W>;
+}
+
+// The resident solve of a factored system whose rows have at most 6 entries on
+// either side of the diagonal and fit in the SMs' shared memory, with the 6 n
+// more work doubles that a.width > 0 stands for; *taken = false and no launch
+// otherwise. As few blocks as hold the rows. It was the faster one at every size
+// measured, 4,096 to 65,536 rows (2.3 to 6 times a solve), so a system that fits
+// always takes it.
 int launch_sweep(const KrylovArgs& a, bool pcg, cudaStream_t s, bool* taken) {
   *taken = false;
-  if (a.precond == 1 || a.width < 1 || a.width > 7 || a.n < 64) return 0;
+  if (a.precond == 1 || a.width < 1 || a.width > 6) return 0;
   int dev = 0, sms = 0, smem = 0;
   MGPU_CUDA(cudaGetDevice(&dev));
   MGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   MGPU_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const int WO = a.width <= 5 ? 4 : 6;
-  const int room = smem - 2048 - sweep_smem(WO, 0, 6 * (kSweepThreads / 32));
-  const int most = std::min(room / sweep_row_bytes(WO) / kSuperRows * kSuperRows, 6 * kSweepThreads);
+  const int W = a.width <= 3 ? 3 : a.width == 4 ? 4 : 6;
+  const long room = smem - 2048 - sweep_smem(W, 0, a.bw);
+  const int most = room > 0 ? (int)(room / sweep_row_bytes(W) / 32 * 32) : 0;
+  // the polling threads keep their rows in a 32-bit mask; places are 16 bits
+  if (most < 256 || a.bw > 32 * 32 * kPollWarps) return 0;
   const int blocks = (a.n + most - 1) / most;
-  const int R = ((a.n + blocks - 1) / blocks + kSuperRows - 1) / kSuperRows * kSuperRows;
-  const int grid = (a.n + R - 1) / R;
-  if (grid > sms || a.n > 10 * 256 * kSuperRows || R + 2l * a.bw > 65535) return 0;
-  int K = (R + kSweepThreads - 1) / kSweepThreads;
-  K = K <= 2 ? K : K <= 4 ? 4 : 6;
-  const int dyn = sweep_smem(WO, R, K * (kSweepThreads / 32));
-  const void* fn = WO == 4 ? sweep_kernel<4>(K, pcg) : sweep_kernel<6>(K, pcg);
+  const int R = ((a.n + blocks - 1) / blocks + 31) / 32 * 32;
+  if (blocks > sms) return 0;
+  const int dyn = (int)sweep_smem(W, R, a.bw);
+  const void* fn = W == 3 ? sweep_kernel<3>(pcg) : W == 4 ? sweep_kernel<4>(pcg) : sweep_kernel<6>(pcg);
   MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   KrylovArgs aa = a;
-  int RR = R, bw = a.bw;
-  void* args[] = {&aa, &RR, &bw};
+  int block = 0, RR = R, vgrid = krylov_grid(a.n, block, pcg ? 0 : 1);
+  void* args[] = {&aa, &RR, &vgrid};
   MGPU_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
-  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSweepThreads), args, (size_t)dyn, s));
+  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3((a.n + R - 1) / R), dim3(kSweepThreads), args, (size_t)dyn, s));
   *taken = true;
   return 0;
 }

@@ -20,21 +20,42 @@ extern int g_cheb_degree;      // the cheb_degree and cheb_ratio tuning keys
 extern double g_cheb_ratio;
 void cheb_params(long n, int& k, double& ratio);  // krylov.cu
 extern int g_prefetch_mb;      // l2_prefetch_mb
+size_t page_floats(int n, int W, const ResidentPlan& plan);  // krylov_resident.cu
 }
 
 using namespace mgpu;
 
 namespace {
 
+// Device buffers of one call: pieces of one allocation of the size that the
+// caller reserved (an allocation and a release for each buffer took most of a
+// small solve's time), anything beyond it on its own.
 struct DevBuf {
   std::vector<void*> p;
+  char* base = nullptr;
+  size_t left = 0;
   ~DevBuf() {
     for (void* q : p) cudaFree(q);
   }
+  int reserve(size_t bytes) {
+    void* q = nullptr;
+    MGPU_CUDA(cudaMalloc(&q, bytes));
+    p.push_back(q);
+    base = (char*)q;
+    left = bytes;
+    return 0;
+  }
   template <typename T>
   int alloc(T*& out, size_t n) {
+    const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+    if (bytes <= left) {
+      out = (T*)base;
+      base += bytes;
+      left -= bytes;
+      return 0;
+    }
     void* q = nullptr;
-    MGPU_CUDA(cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T)));
+    MGPU_CUDA(cudaMalloc(&q, bytes));
     p.push_back(q);
     out = (T*)q;
     return 0;
@@ -53,48 +74,92 @@ struct DevBuf {
     if (rc_ != 0) return rc_;  \
   } while (0)
 
-// Level sets / transposes of an arbitrary CSR pattern (0-based).
+// What the solves need of a host CSR pattern (1-based, columns ascending).
 struct Pattern {
-  std::vector<int> rp, col, diag, mirror, lo_ptr, lo_rows, up_ptr, up_rows;
-  int nlo = 0, nup = 0;
-  bool symmetric = true, full_diag = true;
+  int *rp = nullptr, *col = nullptr, *diag = nullptr, *mirror = nullptr;  // 0-based, on the device
+  int nnz = 0;
+  bool symmetric = false, full_diag = false;
+  int width = 0, bw = 0;  // most entries of a row on one side of the diagonal, largest |column - row|
 };
 
-void analyse(int n, const int32_t* row_ptr, const int32_t* col_idx, Pattern& P) {
-  P.rp.resize(n + 1);
-  for (int i = 0; i <= n; ++i) P.rp[i] = row_ptr[i] - 1;
-  const int nnz = P.rp[n];
-  P.col.resize(nnz);
-  for (int k = 0; k < nnz; ++k) P.col[k] = col_idx[k] - 1;
-  auto find = [&](int i, int j) {
-    for (int k = P.rp[i]; k < P.rp[i + 1]; ++k) {
-      if (P.col[k] == j) return k;
-      if (P.col[k] > j) return -1;
+enum { kNoDiag, kUnpaired, kSide, kFar, kBadColumn, kFlags };
+
+// The 0-based pattern, the diagonal's and the transposed entries' positions;
+// flags: rows without a diagonal entry, entries without a transposed one, the
+// most entries on one side of a diagonal, the largest |column - row|, columns
+// out of range. A thread a row: the searches run along rows of a few entries
+// (on the host they took longer than the solve).
+__global__ void k_csr_pattern(int n, const int* __restrict__ rp1, const int* __restrict__ col1, int* rp, int* col,
+                              int* diag, int* mirror, int* flags) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > n) return;
+  rp[i] = rp1[i] - 1;
+  if (i == n) return;
+  const int b = rp1[i] - 1, e = rp1[i + 1] - 1;
+  int d = -1, lower = 0, upper = 0, far = 0;
+  for (int k = b; k < e; ++k) {
+    const int j = col1[k] - 1;
+    col[k] = j;
+    if (j < 0 || j >= n) {
+      atomicOr(&flags[kBadColumn], 1);
+      continue;
     }
-    return -1;
-  };
-  P.diag.resize(n);
-  for (int i = 0; i < n; ++i) {
-    P.diag[i] = find(i, i);
-    if (P.diag[i] < 0) P.full_diag = false;
+    far = max(far, abs(j - i));
+    lower += j < i;
+    upper += j > i;
+    if (j == i && d < 0) d = k;
+    int m = -1;
+    for (int q = rp1[j] - 1, qe = rp1[j + 1] - 1; q < qe; ++q) {
+      const int c = col1[q] - 1;
+      if (c == i) m = q;
+      if (c >= i) break;
+    }
+    if (m < 0) {
+      atomicOr(&flags[kUnpaired], 1);
+      m = k;
+    }
+    mirror[k] = m;
   }
-  P.mirror.assign(nnz, 0);
-  for (int i = 0; i < n; ++i)
-    for (int k = P.rp[i]; k < P.rp[i + 1]; ++k) {
-      P.mirror[k] = find(P.col[k], i);
-      if (P.mirror[k] < 0) {
-        P.symmetric = false;
-        P.mirror[k] = k;
-      }
-    }
-  if (!P.full_diag) return;
+  diag[i] = d;
+  if (d < 0) atomicOr(&flags[kNoDiag], 1);
+  atomicMax(&flags[kSide], max(lower, upper));
+  atomicMax(&flags[kFar], far);
+}
+
+int load_pattern(int n, const int32_t* row_ptr, const int32_t* col_idx, DevBuf& B, Pattern& P) {
+  P.nnz = row_ptr[n] - 1;
+  int *rp1, *col1, *flags;
+  TRY(B.up(rp1, row_ptr, n + 1));
+  TRY(B.up(col1, col_idx, P.nnz));
+  TRY(B.alloc(P.rp, n + 1));
+  TRY(B.alloc(P.col, P.nnz));
+  TRY(B.alloc(P.diag, n));
+  TRY(B.alloc(P.mirror, P.nnz));
+  TRY(B.alloc(flags, kFlags));
+  MGPU_CUDA(cudaMemset(flags, 0, kFlags * sizeof(int)));
+  k_csr_pattern<<<ceil_div(n + 1, 128), 128>>>(n, rp1, col1, P.rp, P.col, P.diag, P.mirror, flags);
+  MGPU_LAUNCH_CHECK("k_csr_pattern");
+  int h[kFlags];
+  MGPU_CUDA(cudaMemcpy(h, flags, sizeof(h), cudaMemcpyDeviceToHost));
+  if (h[kBadColumn]) {
+    set_error("CSR matrix: a column out of range");
+    return MGPU_E_ARG;
+  }
+  P.full_diag = !h[kNoDiag];
+  P.symmetric = !h[kUnpaired];
+  P.width = std::max(h[kSide], 1);
+  P.bw = h[kFar];
+  return 0;
+}
+
+// The triangular level sets (rows by level, ascending in a level).
+struct Levels {
+  std::vector<int> lo_ptr, lo_rows, up_ptr, up_rows;
+  int nlo = 0, nup = 0;
+};
+
+void level_sets(int n, const int32_t* rp, const int32_t* col, Levels& L) {
   std::vector<int> lev(n, 0);
-  for (int i = 0; i < n; ++i) {
-    int l = 0;
-    for (int k = P.rp[i]; k < P.diag[i]; ++k) l = std::max(l, lev[P.col[k]] + 1);
-    lev[i] = l;
-    P.nlo = std::max(P.nlo, l + 1);
-  }
   auto bucket = [&](int nl, std::vector<int>& ptr, std::vector<int>& rows) {
     ptr.assign(nl + 1, 0);
     for (int i = 0; i < n; ++i) ptr[lev[i] + 1]++;
@@ -103,40 +168,41 @@ void analyse(int n, const int32_t* row_ptr, const int32_t* col_idx, Pattern& P) 
     std::vector<int> f(ptr.begin(), ptr.end() - 1);
     for (int i = 0; i < n; ++i) rows[f[lev[i]]++] = i;
   };
-  bucket(P.nlo, P.lo_ptr, P.lo_rows);
+  for (int i = 0; i < n; ++i) {
+    int l = 0;
+    for (int k = rp[i] - 1; k < rp[i + 1] - 1 && col[k] - 1 < i; ++k) l = std::max(l, lev[col[k] - 1] + 1);
+    lev[i] = l;
+    L.nlo = std::max(L.nlo, l + 1);
+  }
+  bucket(L.nlo, L.lo_ptr, L.lo_rows);
   for (int i = n - 1; i >= 0; --i) {
     int l = 0;
-    for (int k = P.diag[i] + 1; k < P.rp[i + 1]; ++k) l = std::max(l, lev[P.col[k]] + 1);
+    for (int k = rp[i + 1] - 2; k >= rp[i] - 1 && col[k] - 1 > i; --k) l = std::max(l, lev[col[k] - 1] + 1);
     lev[i] = l;
-    P.nup = std::max(P.nup, l + 1);
+    L.nup = std::max(L.nup, l + 1);
   }
-  bucket(P.nup, P.up_ptr, P.up_rows);
+  bucket(L.nup, L.up_ptr, L.up_rows);
 }
 
 // The pressure solver of the mixed and FP64 polynomial forms on a host CSR
 // system: the case's own kernels (k_pcg_mixed / k_pcg_poly64) with the
 // arguments a case would give them, the ELL copy built on the device.
 template <typename V>
-int poly_solve(int n, const Pattern& P, const double* val, const double* b, double* x, double tol, int maxit,
+int poly_solve(int n, const Pattern& P, DevBuf& B, const double* val, const double* b, double* x, double tol, int maxit,
                       int cheb_degree, double cheb_ratio, int* it, double* res, int* ierr) {
-  DevBuf B;
-  const int nnz = P.rp[n];
-  int *drp, *dcol, *ddiag, *dferr;
+  const int nnz = P.nnz;
+  int *drp = P.rp, *dcol = P.col, *ddiag = P.diag, *dferr;
   double *dval, *db, *dx, *dkw, *dpart, *dred;
   V *da, *ddinv, *dw;
   unsigned long long* dbar;
   DevStatus* dst;
   MgpuIterRec* drec;
-  TRY(B.up(drp, P.rp.data(), n + 1));
-  TRY(B.up(dcol, P.col.data(), nnz));
-  TRY(B.up(ddiag, P.diag.data(), n));
   TRY(B.up(dval, val, nnz));
   TRY(B.up(db, b, n));
   TRY(B.up(dx, x, n));
   TRY(B.alloc(dkw, 10 * (size_t)n));
   TRY(B.alloc(dpart, 4 * 4096));
   TRY(B.alloc(dred, (size_t)mixed_red_words(n)));
-  TRY(B.alloc(da, nnz));
   TRY(B.alloc(ddinv, n));
   TRY(B.alloc(dw, 10 * (size_t)n));
   TRY(B.alloc(dbar, 1));
@@ -149,7 +215,8 @@ int poly_solve(int n, const Pattern& P, const double* val, const double* b, doub
   int bw = -1;  // the resident solve exchanges between blocks both ways: symmetric patterns only
   TRY(device_ell(n, drp, dcol, 8, W, ld, ell, alloc, 0, &bw));
   ResidentPlan plan;
-  if (sizeof(V) == 4 && P.symmetric) TRY(plan_resident(n, W, (int)ld, ell, bw, plan, 0));
+  if (sizeof(V) == 4 && P.symmetric) TRY(plan_resident(n, W, (int)ld, ell, bw, plan, dferr, 0));
+  TRY(B.alloc(da, nnz + page_floats(n, W, plan)));
   V* dev = nullptr;
   double* dev64 = nullptr;  // the mixed form's FP64 conjugate-gradient product
   if (ell) {
@@ -222,8 +289,11 @@ int mgpu_krylov_solve(int n, const int32_t* row_ptr, const int32_t* col_idx, con
     set_error("mgpu_krylov_solve: invalid argument");
     return MGPU_E_ARG;
   }
+  DevBuf B;
+  const size_t nz = row_ptr[n] - 1;
+  TRY(B.reserve(40 * nz + 220 * (size_t)n + (1 << 18)));
   Pattern P;
-  analyse(n, row_ptr, col_idx, P);
+  TRY(load_pattern(n, row_ptr, col_idx, B, P));
   const int precond = (method == 0 || method == 4) ? 0 : (method == 2 ? 2 : 1);
   const bool bicg = method == 0 || method == 3;
   *it = 0;
@@ -244,26 +314,23 @@ int mgpu_krylov_solve(int n, const int32_t* row_ptr, const int32_t* col_idx, con
     set_error("mgpu_krylov_solve: IC(0) needs a structurally symmetric pattern");
     return MGPU_E_ARG;
   }
-  DevBuf B;
-  const int nnz = P.rp[n];
-  int *drp, *dcol, *ddiag, *dmir, *dlop, *dlor, *dupp, *dupr, *dferr;
+  Levels L;
+  if (precond != 1) level_sets(n, row_ptr, col_idx, L);
+  const int nnz = P.nnz;
+  int *drp = P.rp, *dcol = P.col, *ddiag = P.diag, *dmir = P.mirror, *dlop, *dlor, *dupp, *dupr, *dferr;
   double *dval, *dfval, *db, *dx, *dkw, *dpart;
   unsigned long long* dbar;
   DevStatus* dst;
   MgpuIterRec* drec;
-  TRY(B.up(drp, P.rp.data(), n + 1));
-  TRY(B.up(dcol, P.col.data(), nnz));
-  TRY(B.up(ddiag, P.diag.data(), n));
-  TRY(B.up(dmir, P.mirror.data(), nnz));
-  TRY(B.up(dlop, P.lo_ptr.data(), P.lo_ptr.size()));
-  TRY(B.up(dlor, P.lo_rows.data(), n));
-  TRY(B.up(dupp, P.up_ptr.data(), P.up_ptr.size()));
-  TRY(B.up(dupr, P.up_rows.data(), n));
+  TRY(B.up(dlop, L.lo_ptr.data(), L.lo_ptr.size()));
+  TRY(B.up(dlor, L.lo_rows.data(), L.lo_rows.size()));
+  TRY(B.up(dupp, L.up_ptr.data(), L.up_ptr.size()));
+  TRY(B.up(dupr, L.up_rows.data(), L.up_rows.size()));
   TRY(B.up(dval, val, nnz));
   TRY(B.alloc(dfval, nnz));
   TRY(B.up(db, b, n));
   TRY(B.up(dx, x, n));
-  TRY(B.alloc(dkw, 10 * (size_t)n));
+  TRY(B.alloc(dkw, 16 * (size_t)n));
   TRY(B.alloc(dpart, 4 * 4096));
   TRY(B.alloc(dbar, 1));
   TRY(B.alloc(dferr, 1));
@@ -295,16 +362,18 @@ int mgpu_krylov_solve(int n, const int32_t* row_ptr, const int32_t* col_idx, con
   a.sh = dkw + 7l * n;
   a.z = dkw + 8l * n;
   a.w = dkw + 9l * n;
-  a.nlev_lo = P.nlo;
+  a.nlev_lo = L.nlo;
   a.lo_ptr = dlop;
   a.lo_rows = dlor;
-  a.nlev_up = P.nup;
+  a.nlev_up = L.nup;
   a.up_ptr = dupp;
   a.up_rows = dupr;
   a.lt_pos = dmir;
   a.tol = tol;
   a.maxit = maxit;
   a.precond = precond;
+  a.width = P.width;
+  a.bw = P.bw;
   a.zero_x = 0;
   a.mpi_mode = norm_mode ? 1 : 0;
   a.partials = dpart;
@@ -343,8 +412,11 @@ int mgpu_pcg_poly_solve(int n, const int32_t* row_ptr, const int32_t* col_idx, c
     set_error("mgpu_pcg_poly_solve: invalid argument");
     return MGPU_E_ARG;
   }
+  DevBuf B;
+  const size_t nz = row_ptr[n] - 1;
+  TRY(B.reserve(32 * nz + 520 * (size_t)n + (1 << 18)));
   Pattern P;
-  analyse(n, row_ptr, col_idx, P);
+  TRY(load_pattern(n, row_ptr, col_idx, B, P));
   *it = 0;
   *res = 0.0;
   *ierr = 0;
@@ -355,8 +427,8 @@ int mgpu_pcg_poly_solve(int n, const int32_t* row_ptr, const int32_t* col_idx, c
   int k = cheb_degree;
   double ratio = g_cheb_ratio;
   if (k <= 0) cheb_params(n, k, ratio);  // the tuning keys, as a case's pressure solve of n rows
-  return precision == MGPU_PREC_MIXED ? poly_solve<float>(n, P, val, b, x, tol, maxit, k, ratio, it, res, ierr)
-                                      : poly_solve<double>(n, P, val, b, x, tol, maxit, k, ratio, it, res, ierr);
+  return precision == MGPU_PREC_MIXED ? poly_solve<float>(n, P, B, val, b, x, tol, maxit, k, ratio, it, res, ierr)
+                                      : poly_solve<double>(n, P, B, val, b, x, tol, maxit, k, ratio, it, res, ierr);
 }
 
 int mgpu_csr_matvec(int n, const int32_t* row_ptr, const int32_t* col_idx, const double* val, const double* x,
