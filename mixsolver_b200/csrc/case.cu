@@ -687,16 +687,12 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
     MGPU_CUDA(cudaMemcpyAsync(d.ramp, one, sizeof(one), cudaMemcpyHostToDevice, c->stream));
   }
   if ((e = ensure_recs(c, 64))) return fail(e);
-  if (!poly) {
-    int wide = 0;
-    if ((e = device_row_extent(d.N, d.row_ptr, d.col, wide, d.bw, d.width, (int*)d.partials, c->stream)))
-      return fail(e);
-  }
+  int far = 0;  // largest |column - row|
   if (poly) {
     // column-major ELL copy of the pattern for the polynomial forms' SpMV (rows of at most 8 entries)
-    int w = 0, bw = 0, *ell = nullptr;
+    int w = 0, *ell = nullptr;
     long ld = 0;
-    if ((e = device_ell(d.N, d.row_ptr, d.col, 8, w, ld, ell, keep, c->stream, &bw))) return fail(e);
+    if ((e = device_ell(d.N, d.row_ptr, d.col, 8, w, ld, ell, keep, c->stream, &far))) return fail(e);
     if (ell) {
       d.ell_col = ell;
       // values zero in the padding rows
@@ -707,13 +703,10 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
       if (ctrl->precision == MGPU_PREC_MIXED) {
         if ((e = c->alloc(d.ell_val, (size_t)w * ld))) return fail(e);
         MGPU_CUDA(cudaMemsetAsync(d.ell_val, 0, sizeof(float) * (size_t)w * ld, c->stream));
-        if ((e = plan_resident(d.N, w, (int)ld, ell, bw, d.plan, d.ferr, c->stream))) return fail(e);
       }
       d.ell_w = w;
       d.ell_ld = (int)ld;
     }
-    // the pages of a larger system's pressure solve follow its CSR values
-    if (ctrl->precision == MGPU_PREC_MIXED && (e = c->alloc(d.a32, d.nnz + page_floats(d.N, w, d.plan)))) return fail(e);
   }
   // geometry (device), scratch for the node arrays and provisional centres
   std::vector<int> fptr_h(hm.fptr.begin(), hm.fptr.end());
@@ -817,6 +810,19 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
   MGPU_CUDA(cudaMemsetAsync(d.bar, 0, sizeof(unsigned long long), c->stream));
   if ((e = launch_fill(d.apc, N, 1.0, c->stream))) return fail(e);
   MGPU_CUDA(cudaStreamSynchronize(c->stream));
+  // how the solves divide the system; here, after the set-up's buffers have gone
+  // back (a wait between them hands their memory to the driver and the next
+  // allocation maps it again)
+  if (!poly) {
+    int wide = 0;
+    if ((e = device_row_extent(d.N, d.row_ptr, d.col, wide, d.bw, d.width, (int*)d.partials, c->stream)))
+      return fail(e);
+  }
+  if (ctrl->precision == MGPU_PREC_MIXED) {
+    if ((e = plan_resident(d.N, d.ell_w, d.ell_ld, d.ell_col, far, d.plan, d.ferr, c->stream))) return fail(e);
+    // the pages of a larger system's pressure solve follow its CSR values
+    if ((e = c->alloc(d.a32, d.nnz + page_floats(d.N, d.ell_w, d.plan)))) return fail(e);
+  }
   // scalars needing a sequential pass: flux_ref (group/face order) and the
   // smallest vol**(1/3) (CFL estimate); computed once on the host
   std::vector<double> area(F), vol(N);

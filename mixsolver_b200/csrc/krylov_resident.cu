@@ -1296,7 +1296,8 @@ int launch_resident(const KrylovArgs& a, const MixedArgs& m, bool pcg, cudaStrea
   const int dyn = resident_smem(WC, R, m.plan.bw, m.plan.words, K * (T / 32));
   const int which = paged ? kPcgPaged : pcg ? kPcg : kBicg;
   const void* fn = WC == 5 ? resident_kernel<5>(K, which) : resident_kernel<7>(K, which);
-  MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  // the same limit on every call: another thread may be launching the kernel for another system
+  MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - kStaticSmem));
   KrylovArgs aa = a;
   MixedArgs mm = m;
   int RR = R, words = m.plan.words;

@@ -744,7 +744,8 @@ int launch_sweep(const KrylovArgs& a, bool pcg, cudaStream_t s, bool* taken) {
   if (blocks > sms) return 0;
   const int dyn = (int)sweep_smem(W, R, a.bw);
   const void* fn = W == 3 ? sweep_kernel<3>(pcg) : W == 4 ? sweep_kernel<4>(pcg) : sweep_kernel<6>(pcg);
-  MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  // the same limit on every call: another thread may be launching the kernel for another system
+  MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 2048));
   KrylovArgs aa = a;
   int block = 0, RR = R, vgrid = krylov_grid(a.n, block, pcg ? 0 : 1);
   void* args[] = {&aa, &RR, &vgrid};
