@@ -378,9 +378,12 @@ int mgpu_cg_jacobi_noalloc(int n, const int32_t* d_row_ptr, const int32_t* d_col
  * (the FP64 polynomial form 2-5), the register budget sized to match,
  * default 5), "batch_blocks_per_sm" (the
  * same for batched lanes, default 4; set before building a batch),
- * "spin_limit" (failed polls
- * after which a grid-barrier wait gives up, 0 = the built-in bound of about
- * 2 s; for tests of the timeout path), "gather_faces" (assembly kernels: the
+ * "resident_sms" (SMs that the division of a mixed system over the SMs'
+ * shared memory counts on, 0, the default: all; otherwise a system too large
+ * for that many is solved in turns whether or not that pays; set before
+ * creating a case; for tests of the division of large systems on small ones),
+ * "spin_limit" (failed polls after which a grid-barrier wait gives up, 0 = the
+ * built-in bound of about 2 s; for tests of the timeout path), "gather_faces" (assembly kernels: the
  * faces of a cell whose loads a thread issues before summing, 1, 2, 3 or 6
  * (4 and 5 take 3); 0, the default, gives each kernel its measured best;
  * results are the same bits for every value), "barrier_poll_ns" (sleep between two

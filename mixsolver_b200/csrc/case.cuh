@@ -73,11 +73,11 @@ struct KrylovArgs {
 
 // How a system is divided for its resident solves (krylov_resident.cu): rows of
 // a block (0: no resident solve), most 32-row words a block reads of
-// other blocks, largest |column - row|; steps > 0: the system is larger than
-// the SMs' shared memory and its pressure solve takes the blocks in turns,
-// `steps` polynomial steps a turn.
+// other blocks, largest |column - row|, blocks; steps > 0: the system is larger
+// than the SMs' shared memory and its pressure solve takes pages of that many
+// rows in turns, `steps` polynomial steps a turn.
 struct ResidentPlan {
-  int rows = 0, words = 0, bw = 0, steps = 0;
+  int rows = 0, words = 0, bw = 0, blocks = 0, steps = 0;
 };
 
 // Data of a polynomial-preconditioned solve in working precision V: the

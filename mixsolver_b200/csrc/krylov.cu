@@ -64,6 +64,7 @@ void cheb_params(long n, int& k, double& ratio) {
 }
 unsigned g_spin_limit = 0; // polls before a bounded barrier wait gives up (0: kSpinLimit, ~2 s)
 unsigned g_poll_ns = 100;  // sleep between the polls of a barrier wait (ns)
+int g_resident_sms = 0;    // SMs that the division of a mixed system over shared memory counts on (0: all)
 int g_mixed_occ = 5;       // mixed kernels: resident blocks per SM (2-8; FP64 polynomial 2-5)
 int g_gather_faces = 0;    // assembly gathers: faces whose loads a thread issues together (0: per kernel)
 int g_batch_occ = 4;       // batched lane kernel: resident blocks per SM (2-5)
@@ -779,6 +780,8 @@ int set_tuning(const char* key, int value) {
     g_batch_reserve = value;
   } else if (k == "l2_prefetch_mb" && value >= 0) {
     g_prefetch_mb = value;
+  } else if (k == "resident_sms" && value >= 0) {
+    g_resident_sms = value;
   } else if (k == "mixed_blocks_per_sm" && value >= 2 && value <= 8) {
     g_mixed_occ = value;
   } else if (k == "batch_blocks_per_sm" && value >= 2 && value <= 5) {
@@ -823,6 +826,8 @@ int get_tuning(const char* key, int* value) {
     *value = g_batch_reserve;
   } else if (k == "l2_prefetch_mb") {
     *value = g_prefetch_mb;
+  } else if (k == "resident_sms") {
+    *value = g_resident_sms;
   } else if (k == "mixed_blocks_per_sm") {
     *value = g_mixed_occ;
   } else if (k == "batch_blocks_per_sm") {

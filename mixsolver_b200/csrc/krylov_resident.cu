@@ -39,6 +39,7 @@
 #include "krylov_poly.cuh"
 
 namespace mgpu {
+extern int g_resident_sms;  // krylov.cu: the resident_sms tuning key
 namespace {
 
 // Blocks of 256 threads, two per SM, or of 512, one per SM; 128 registers each.
@@ -1149,11 +1150,26 @@ __global__ void k_halo_words(int n, int W, int ld, const int* __restrict__ ell_c
 
 enum { kBicg = 0, kPcg = 1, kPcgPaged = 2 };
 
+// Threads of a block of R rows (a multiple of 256) and the rows of a thread,
+// one of the compiled counts.
+constexpr int block_threads(int R) { return R > kPairRows ? 512 : 256; }
+constexpr int thread_rows(int R) {
+  const int K = (R + block_threads(R) - 1) / block_threads(R);
+  return K <= 5 ? K : K <= 7 ? 7 : 9;
+}
+
+constexpr int kPageMin = 5, kPageMax = 9;  // super-chunks of a page
+constexpr int kPageThreadRows = thread_rows(kPageMin * kSuperRows);  // and the rows of its threads, at least
+static_assert(block_threads(kPageMax * kSuperRows) == 256 && thread_rows(kPageMax * kSuperRows) == 9,
+              "k_pcg_paged is compiled for blocks of 256 threads of up to 9 rows");
+
+// The kernel of a solve; null when none is compiled for these rows a thread.
 template <int WC, int K>
 const void* resident_kernel_k(int which) {
-  if constexpr (K >= 7)
-    if (which == kPcgPaged) return (const void*)k_pcg_paged<WC, K>;
-  return which == kPcg ? (const void*)k_pcg_resident<WC, K> : (const void*)k_bicgstab_resident<WC, K>;
+  if (which == kBicg) return (const void*)k_bicgstab_resident<WC, K>;
+  if (which == kPcg) return (const void*)k_pcg_resident<WC, K>;
+  if constexpr (K >= kPageThreadRows) return (const void*)k_pcg_paged<WC, K>;
+  return nullptr;
 }
 
 template <int WC>
@@ -1165,7 +1181,8 @@ const void* resident_kernel(int K, int which) {
     case 4: return resident_kernel_k<WC, 4>(which);
     case 5: return resident_kernel_k<WC, 5>(which);
     case 7: return resident_kernel_k<WC, 7>(which);
-    default: return resident_kernel_k<WC, 9>(which);
+    case 9: return resident_kernel_k<WC, 9>(which);
+    default: return nullptr;
   }
 }
 
@@ -1179,25 +1196,13 @@ int device_limits(int& sms, int& smem_sm) {
   return 0;
 }
 
-// Threads of a block of R rows (a multiple of 256) and the rows of a thread,
-// one of the compiled counts.
-void resident_shape(int R, int& T, int& K) {
-  T = R > kPairRows ? 512 : 256;
-  K = (R + T - 1) / T;
-  if (K > 5) K = K <= 7 ? 7 : 9;
-}
-
-}  // namespace
-
-namespace {
 // The most halo words of a block when the rows are cut into blocks of R, and
 // whether such a block fits: rows and window in an SM's shared memory, window
 // offsets in 16 bits.
 int fit_rows(int n, int W, int ld, const int* ell_col, int bw, int R, int room, int& words, bool& fits, int* most,
              cudaStream_t s) {
   const int WC = W <= 5 ? 5 : 7, flags = 4 * resident_window_words(R, bw);
-  int T, K;
-  resident_shape(R, T, K);
+  const int T = block_threads(R), K = thread_rows(R);
   fits = false;
   if (resident_smem(WC, R, bw, 0, K * (T / 32)) > room || flags > 48 * 1024) return 0;
   MGPU_CUDA(cudaMemsetAsync(most, 0, sizeof(int), s));
@@ -1219,6 +1224,7 @@ int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan
   if (!ell_col || W > 7 || bw < 0 || n < kSuperRows / 4) return 0;
   int sms = 0, smem = 0;
   if (int e = device_limits(sms, smem)) return e;
+  if (g_resident_sms > 0) sms = std::min(sms, g_resident_sms);
   const int nsc = (n + kSuperRows - 1) / kSuperRows;
   if (nsc > 256 * kSumGroups) return 0;
   const int pair = (nsc + 2 * sms - 1) / (2 * sms), single = (nsc + sms - 1) / sms;
@@ -1229,6 +1235,7 @@ int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan
     plan.rows = R;
     plan.words = words;
     plan.bw = bw;
+    plan.blocks = std::min((n + R - 1) / R, 2 * sms);
   };
   // two blocks of 256 threads per SM up to 6 super-chunks each (one PCG
   // iteration of 42,253 rows 42 -> 35 us against one block of 512), then one of
@@ -1251,7 +1258,7 @@ int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan
   // streamed pass took about 2.3 G page-step times, so the turns are used while
   // they promise a fifth less than that.
   const int most = 2 * sms;
-  for (int sc = 9; sc >= 5 && !fits; --sc) {
+  for (int sc = kPageMax; sc >= kPageMin && !fits; --sc) {
     const int R = sc * kSuperRows;
     if (R * (long)most > n) continue;  // a page for every block at least
     if (int e = fit_rows(n, W, ld, ell_col, bw, R, half, words, fits, scratch, s)) return e;
@@ -1265,7 +1272,7 @@ int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan
         plan.steps = st;
       }
     }
-    if (best <= 0.0 || most / best > 0.8 * 2.3) {
+    if (best <= 0.0 || (g_resident_sms == 0 && most / best > 0.8 * 2.3)) {
       plan = ResidentPlan{};
       return 0;
     }
@@ -1281,30 +1288,31 @@ size_t page_floats(int n, int W, const ResidentPlan& plan) {
 }
 
 // The resident solve of a planned system; *taken = false and no launch when
-// there is no plan, no polynomial to apply, or turns are planned (pressure only). A planned system always takes it: from 64 rows (the smallest
-// planned) to the largest that fits, about 570,000 rows of 7 entries, it measured
-// faster than the streaming kernel.
+// there is no plan, no polynomial to apply, no kernel for the plan's rows, or
+// turns are planned (pressure only). A planned system always takes it: from 64
+// rows (the smallest planned) to the largest that fits, about 570,000 rows of 7
+// entries, it measured faster than the streaming kernel.
 int launch_resident(const KrylovArgs& a, const MixedArgs& m, bool pcg, cudaStream_t s, bool* taken) {
   *taken = false;
   if (m.plan.rows <= 0 || (pcg && (!m.ell64 || m.cheb_k < 2 || m.cheb_k > 64))) return 0;
   const bool paged = m.plan.steps > 0;
   if (paged && !pcg) return 0;
   const int R = m.plan.rows, WC = m.ell_w <= 5 ? 5 : 7;
-  int T, K, sms = 0, smem = 0;
-  if (int e = device_limits(sms, smem)) return e;
-  resident_shape(R, T, K);
+  const int T = block_threads(R), K = thread_rows(R);
   const int dyn = resident_smem(WC, R, m.plan.bw, m.plan.words, K * (T / 32));
   const int which = paged ? kPcgPaged : pcg ? kPcg : kBicg;
   const void* fn = WC == 5 ? resident_kernel<5>(K, which) : resident_kernel<7>(K, which);
+  if (!fn) return 0;
+  int sms = 0, smem = 0;
+  if (int e = device_limits(sms, smem)) return e;
   // the same limit on every call: another thread may be launching the kernel for another system
   MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - kStaticSmem));
   KrylovArgs aa = a;
   MixedArgs mm = m;
   int RR = R, words = m.plan.words;
   void* args[] = {&aa, &mm, &RR, &words};  // the paged kernel takes the first two
-  const int grid = std::min((a.n + R - 1) / R, paged ? 2 * sms : 1 << 30);
   MGPU_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
-  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(T), args, (size_t)dyn, s));
+  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3(m.plan.blocks), dim3(T), args, (size_t)dyn, s));
   *taken = true;
   return 0;
 }
