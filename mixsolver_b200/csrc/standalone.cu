@@ -79,16 +79,20 @@ struct Pattern {
   int *rp = nullptr, *col = nullptr, *diag = nullptr, *mirror = nullptr;  // 0-based, on the device
   int nnz = 0;
   bool symmetric = false, full_diag = false;
-  int width = 0, bw = 0;  // most entries of a row on one side of the diagonal, largest |column - row|
+  // most entries of a row on one side of the diagonal (0: some row's columns do not ascend, and its entries
+  // before and after the diagonal need not be those of smaller and larger columns), largest |column - row|
+  int width = 0, bw = 0;
 };
 
-enum { kNoDiag, kUnpaired, kSide, kFar, kBadColumn, kFlags };
+enum { kNoDiag, kUnpaired, kUnsorted, kSide, kFar, kBadColumn, kFlags };
 
 // The 0-based pattern, the diagonal's and the transposed entries' positions;
-// flags: rows without a diagonal entry, entries without a transposed one, the
-// most entries on one side of a diagonal, the largest |column - row|, columns
-// out of range. A thread a row: the searches run along rows of a few entries
-// (on the host they took longer than the solve).
+// flags: rows without a diagonal entry, entries without a transposed one, rows
+// whose columns do not ascend, the most entries on one side of a diagonal, the
+// largest |column - row|, columns out of range. A search ends at the first
+// larger column, so an entry after one is not found. A thread a row: the
+// searches run along rows of a few entries (on the host they took longer than
+// the solve).
 __global__ void k_csr_pattern(int n, const int* __restrict__ rp1, const int* __restrict__ col1, int* rp, int* col,
                               int* diag, int* mirror, int* flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -96,7 +100,8 @@ __global__ void k_csr_pattern(int n, const int* __restrict__ rp1, const int* __r
   rp[i] = rp1[i] - 1;
   if (i == n) return;
   const int b = rp1[i] - 1, e = rp1[i + 1] - 1;
-  int d = -1, lower = 0, upper = 0, far = 0;
+  int d = -1, lower = 0, upper = 0, far = 0, prev = -1;
+  bool past = false, sorted = true;  // past: a column after the diagonal has been met
   for (int k = b; k < e; ++k) {
     const int j = col1[k] - 1;
     col[k] = j;
@@ -107,7 +112,10 @@ __global__ void k_csr_pattern(int n, const int* __restrict__ rp1, const int* __r
     far = max(far, abs(j - i));
     lower += j < i;
     upper += j > i;
-    if (j == i && d < 0) d = k;
+    if (j == i && d < 0 && !past) d = k;
+    past = past || j > i;
+    sorted = sorted && j > prev;
+    prev = j;
     int m = -1;
     for (int q = rp1[j] - 1, qe = rp1[j + 1] - 1; q < qe; ++q) {
       const int c = col1[q] - 1;
@@ -122,6 +130,7 @@ __global__ void k_csr_pattern(int n, const int* __restrict__ rp1, const int* __r
   }
   diag[i] = d;
   if (d < 0) atomicOr(&flags[kNoDiag], 1);
+  if (!sorted) atomicOr(&flags[kUnsorted], 1);
   atomicMax(&flags[kSide], max(lower, upper));
   atomicMax(&flags[kFar], far);
 }
@@ -147,12 +156,13 @@ int load_pattern(int n, const int32_t* row_ptr, const int32_t* col_idx, DevBuf& 
   }
   P.full_diag = !h[kNoDiag];
   P.symmetric = !h[kUnpaired];
-  P.width = std::max(h[kSide], 1);
+  P.width = h[kUnsorted] ? 0 : std::max(h[kSide], 1);
   P.bw = h[kFar];
   return 0;
 }
 
-// The triangular level sets (rows by level, ascending in a level).
+// The triangular level sets (rows by level, ascending in a level); each row has
+// its diagonal entry before any larger column.
 struct Levels {
   std::vector<int> lo_ptr, lo_rows, up_ptr, up_rows;
   int nlo = 0, nup = 0;
@@ -170,14 +180,15 @@ void level_sets(int n, const int32_t* rp, const int32_t* col, Levels& L) {
   };
   for (int i = 0; i < n; ++i) {
     int l = 0;
-    for (int k = rp[i] - 1; k < rp[i + 1] - 1 && col[k] - 1 < i; ++k) l = std::max(l, lev[col[k] - 1] + 1);
+    for (int k = rp[i] - 1; col[k] - 1 < i; ++k) l = std::max(l, lev[col[k] - 1] + 1);
     lev[i] = l;
     L.nlo = std::max(L.nlo, l + 1);
   }
   bucket(L.nlo, L.lo_ptr, L.lo_rows);
   for (int i = n - 1; i >= 0; --i) {
-    int l = 0;
-    for (int k = rp[i + 1] - 2; k >= rp[i] - 1 && col[k] - 1 > i; --k) l = std::max(l, lev[col[k] - 1] + 1);
+    int l = 0, k = rp[i] - 1;
+    while (col[k] - 1 != i) ++k;
+    for (++k; k < rp[i + 1] - 1; ++k) l = std::max(l, lev[col[k] - 1] + 1);
     lev[i] = l;
     L.nup = std::max(L.nup, l + 1);
   }
