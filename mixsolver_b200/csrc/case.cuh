@@ -77,7 +77,8 @@ struct KrylovArgs {
 // than the SMs' shared memory and its pressure solve takes pages of that many
 // rows in turns, `steps` polynomial steps a turn.
 struct ResidentPlan {
-  int rows = 0, words = 0, bw = 0, blocks = 0, steps = 0;
+  int rows = 0, words = 0, bw = 0;
+  short steps = 0, blocks = 0;
 };
 
 // Data of a polynomial-preconditioned solve in working precision V: the
