@@ -383,12 +383,15 @@ int mgpu_cg_jacobi_noalloc(int n, const int32_t* d_row_ptr, const int32_t* d_col
  * for that many is solved in turns whether or not that pays; set before
  * creating a case; for tests of the division of large systems on small ones),
  * "spin_limit" (failed polls after which a grid-barrier wait gives up, 0 = the
- * built-in bound of about 2 s; for tests of the timeout path), "gather_faces" (assembly kernels: the
+ * built-in bound of about 2 s; for tests of the timeout path),
+ * "exchange_spin_limit" (the same for a wait for a value of another block in
+ * the solves that exchange values), "gather_faces" (assembly kernels: the
  * faces of a cell whose loads a thread issues before summing, 1, 2, 3 or 6
  * (4 and 5 take 3); 0, the default, gives each kernel its measured best;
  * results are the same bits for every value), "barrier_poll_ns" (sleep between two
  * polls of a grid-barrier wait, 0-10000 ns, default 100; 0 polls back to back
- * and backs off by 64 ns after 256 polls). */
+ * and backs off by 64 ns after 256 polls; the sums of the solves that exchange
+ * values always poll back to back). */
 int mgpu_set_tuning(const char* key, int value);
 /* The value in effect of a mgpu_set_tuning key (every key but stream_pool),
  * e.g. the Chebyshev degree a byte model of the mixed pressure solve needs. */

@@ -40,12 +40,27 @@ __device__ __forceinline__ void ld_pair(const u64* p, u64& a, u64& b) {
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
 }
 
-constexpr unsigned kHaloSpins = 1u << 22;  // failed polls (each a trip to L2) before a wait gives up, ~2 s
+// Failed polls before a wait for other blocks gives up, ~2 s: each is a trip to
+// L2, or a shared-memory load where another warp of the block brings the value.
+constexpr unsigned kHaloSpins = 1u << 22;
+constexpr unsigned kSharedSpins = 1u << 26;
 
-// One more failed poll of a wait: false once the wait has run out or another
+// The limits of a launch, kernel arguments: the sums' barrier takes the spin_limit
+// tuning key, values take exchange_spin_limit. Polls follow one another at once:
+// with the limits in shared memory and the sleep of vg_sync (barrier_poll_ns)
+// between the barrier's polls a pass of the 42,253-row channel took 4.67 ms, 4.56 so.
+struct WaitLimits {
+  unsigned barrier, value, shared;
+};
+inline WaitLimits wait_limits(unsigned spin_limit, unsigned exchange_limit) {
+  return {spin_limit ? spin_limit : kHaloSpins, exchange_limit ? exchange_limit : kHaloSpins,
+          exchange_limit ? exchange_limit : kSharedSpins};
+}
+
+// One more failed poll of a wait, of the polls left: false once none is or another
 // block has flagged a timeout.
-__device__ __forceinline__ bool keep_polling(unsigned& spins, DevStatus* st) {
-  if ((++spins & 1023u) == 0u && (ld_acquire_i32(&st->timeout) != 0 || spins >= kHaloSpins)) {
+__device__ __forceinline__ bool keep_polling(unsigned& left, DevStatus* st) {
+  if ((--left & 1023u) == 0u && (left == 0u || ld_acquire_i32(&st->timeout) != 0)) {
     atomicExch(&st->timeout, 1);
     return false;
   }
@@ -77,11 +92,11 @@ __device__ __forceinline__ void vg_arrive(const VGrid& g) {
   if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(g.bar) : "memory");
 }
 
-__device__ __forceinline__ bool vg_wait(VGrid& g, DevStatus* st) {
+__device__ __forceinline__ bool vg_wait(VGrid& g, unsigned limit, DevStatus* st) {
   bool ok = true;
   if (threadIdx.x == 0) {
-    unsigned spins = 0;
-    while (ok && ld_acquire_u64(g.bar) < g.next) ok = keep_polling(spins, st);
+    unsigned left = limit;
+    while (ok && ld_acquire_u64(g.bar) < g.next) ok = keep_polling(left, st);
   }
   g.next += (u64)g.nb;
   return __syncthreads_and(ok) != 0;
@@ -127,7 +142,7 @@ __device__ __forceinline__ bool total_wait(State& S, VGrid& g, DevStatus* st, do
   const unsigned half = S.rseq & 1u;
   const int nsc = S.nsc, ng = (nsc + 255) >> 8;
   const double* sums = S.sums + half * 2l * nsc;
-  if (!vg_wait(g, st)) return false;
+  if (!vg_wait(g, S.waits.barrier, st)) return false;
   for (int k = warp; k < ng * NQ; k += nw) {
     const int q = NQ == 1 ? 0 : k & 1, gk = NQ == 1 ? k : k >> 1;
     const double* p = sums + (long)q * nsc;

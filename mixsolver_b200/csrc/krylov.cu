@@ -63,6 +63,7 @@ void cheb_params(long n, int& k, double& ratio) {
   ratio = large ? g_cheb_ratio_large : g_cheb_ratio;
 }
 unsigned g_spin_limit = 0; // polls before a bounded barrier wait gives up (0: kSpinLimit, ~2 s)
+unsigned g_exchange_limit = 0;  // polls before a wait for a value of another block gives up (0: kHaloSpins, ~2 s)
 unsigned g_poll_ns = 100;  // sleep between the polls of a barrier wait (ns)
 int g_resident_sms = 0;    // SMs that the division of a mixed system over shared memory counts on (0: all)
 int g_mixed_occ = 5;       // mixed kernels: resident blocks per SM (2-8; FP64 polynomial 2-5)
@@ -788,6 +789,8 @@ int set_tuning(const char* key, int value) {
     g_batch_occ = value;
   } else if (k == "spin_limit" && value >= 0) {
     g_spin_limit = (unsigned)value;
+  } else if (k == "exchange_spin_limit" && value >= 0) {
+    g_exchange_limit = (unsigned)value;
   } else if (k == "gather_faces" && value >= 0 && value <= 6) {
     g_gather_faces = value;
   } else if (k == "barrier_poll_ns" && value >= 0 && value <= 10000) {
@@ -834,6 +837,8 @@ int get_tuning(const char* key, int* value) {
     *value = g_batch_occ;
   } else if (k == "spin_limit") {
     *value = (int)g_spin_limit;
+  } else if (k == "exchange_spin_limit") {
+    *value = (int)g_exchange_limit;
   } else if (k == "gather_faces") {
     *value = g_gather_faces;
   } else if (k == "barrier_poll_ns") {

@@ -39,7 +39,9 @@
 #include "krylov_poly.cuh"
 
 namespace mgpu {
-extern int g_resident_sms;  // krylov.cu: the resident_sms tuning key
+extern int g_resident_sms;         // krylov.cu: the resident_sms tuning key
+extern unsigned g_spin_limit;      // spin_limit
+extern unsigned g_exchange_limit;  // exchange_spin_limit
 namespace {
 
 // Blocks of 256 threads, two per SM, or of 512, one per SM; 128 registers each.
@@ -66,6 +68,7 @@ struct Resident {
   u64* ll;               // exchange words (2 parities of n)
   double* sums;          // super-chunk sums (2 halves x 2 sums x nsc)
   int hpw;               // halo words per warp, rounded up
+  WaitLimits waits;
   int hrow[kHaloRegs];   // the rows this lane polls for the warp's first halo words
 };
 
@@ -173,13 +176,13 @@ __device__ __forceinline__ bool halo_fetch(const Resident<WC>& S, const u64* llb
   u64 v[HB];
 #pragma unroll
   for (int q = 0; q < HB; ++q) v[q] = ld_word(llb + row[q]);
-  unsigned spins = 0;
+  unsigned left = S.waits.value;
   while (true) {
     unsigned bad = 0u;
 #pragma unroll
     for (int q = 0; q < HB; ++q) bad |= (unsigned)(v[q] >> 32) ^ seq;
     if (bad == 0u) break;
-    if (!keep_polling(spins, st)) return false;
+    if (!keep_polling(left, st)) return false;
 #pragma unroll
     for (int q = 0; q < HB; ++q)
       if ((unsigned)(v[q] >> 32) != seq) v[q] = ld_word(llb + row[q]);
@@ -582,8 +585,9 @@ __device__ __forceinline__ void resident_pcg(const KrylovArgs& a, const MixedArg
 // b = 0, or a zero diagonal with code diag_code).
 template <int WC, int K, bool PCG>
 __device__ __forceinline__ bool resident_begin(const KrylovArgs& a, const MixedArgs& m, VGrid& g, Resident<WC>& S,
-                                               int R, int nhw_max, int diag_code, double& bnrm) {
+                                               WaitLimits waits, int R, int nhw_max, int diag_code, double& bnrm) {
   const int n = a.n;
+  S.waits = waits;
   S.n = n;
   S.R = R;
   S.nb = g.nb;
@@ -610,13 +614,14 @@ __device__ __forceinline__ bool resident_begin(const KrylovArgs& a, const MixedA
 
 // nhw_max: the halo words the shared memory was sized for.
 template <int WC, int K>
-__global__ void __launch_bounds__(kResidentThreads, 1) k_pcg_resident(KrylovArgs a, MixedArgs m, int R, int nhw_max) {
+__global__ void __launch_bounds__(kResidentThreads, 1) k_pcg_resident(KrylovArgs a, MixedArgs m, WaitLimits waits,
+                                                                       int R, int nhw_max) {
   if (a.st->abort) return;
   VGrid g = whole_grid(a.bar, a.partials, true);
   const int T = blockDim.x, tid = threadIdx.x;
   Resident<WC> S;
   double bnrm;
-  if (!resident_begin<WC, K, true>(a, m, g, S, R, nhw_max, 2, bnrm)) return;
+  if (!resident_begin<WC, K, true>(a, m, g, S, waits, R, nhw_max, 2, bnrm)) return;
   // Gershgorin bound of D^-1 A (a maximum is exact in any order), b - A x
   double gm = 0.0;
 #pragma unroll
@@ -676,7 +681,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // of exchange (1.9 in the resident solve: here L2 also carries the pages), a turn
 // 4.8 us to load.
 template <int WC, int K>
-__global__ void __launch_bounds__(256, 2) k_pcg_paged(KrylovArgs a, MixedArgs m) {
+__global__ void __launch_bounds__(256, 2) k_pcg_paged(KrylovArgs a, MixedArgs m, WaitLimits waits) {
   if (a.st->abort) return;
   VGrid g = whole_grid(a.bar, a.partials, true);
   const int n = a.n, T = blockDim.x, tid = threadIdx.x, R = m.plan.rows, W = m.ell_w, ld = m.ell_ld;
@@ -685,6 +690,7 @@ __global__ void __launch_bounds__(256, 2) k_pcg_paged(KrylovArgs a, MixedArgs m)
   const long pstep = page_bytes(WC, R, m.plan.words);
   const int warp = tid >> 5, nw = T >> 5;
   Resident<WC> S;
+  S.waits = waits;
   S.n = n;
   S.R = R;
   S.nb = npages;
@@ -985,13 +991,14 @@ __global__ void __launch_bounds__(256, 2) k_pcg_paged(KrylovArgs a, MixedArgs m)
 // registers, one exchange for each of the two products, the same recurrences,
 // sums and decisions.
 template <int WC, int K>
-__global__ void __launch_bounds__(kResidentThreads, 1) k_bicgstab_resident(KrylovArgs a, MixedArgs m, int R, int nhw_max) {
+__global__ void __launch_bounds__(kResidentThreads, 1) k_bicgstab_resident(KrylovArgs a, MixedArgs m, WaitLimits waits,
+                                                                            int R, int nhw_max) {
   if (a.st->abort) return;
   VGrid g = whole_grid(a.bar, a.partials, true);
   const int T = blockDim.x, tid = threadIdx.x;
   Resident<WC> S;
   double bnrm;
-  if (!resident_begin<WC, K, false>(a, m, g, S, R, nhw_max, 12, bnrm)) return;
+  if (!resident_begin<WC, K, false>(a, m, g, S, waits, R, nhw_max, 12, bnrm)) return;
   float r[K], r0[K], p[K], v[K], d[K];
   int total = 0, ierr = 0;
   double res = 0.0;
@@ -1310,7 +1317,8 @@ int launch_resident(const KrylovArgs& a, const MixedArgs& m, bool pcg, cudaStrea
   KrylovArgs aa = a;
   MixedArgs mm = m;
   int RR = R, words = m.plan.words;
-  void* args[] = {&aa, &mm, &RR, &words};  // the paged kernel takes the first two
+  WaitLimits waits = wait_limits(g_spin_limit, g_exchange_limit);
+  void* args[] = {&aa, &mm, &waits, &RR, &words};  // the paged kernel takes the first three
   MGPU_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
   MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3(m.plan.blocks), dim3(T), args, (size_t)dyn, s));
   *taken = true;

@@ -35,6 +35,8 @@
 #include "exchange.cuh"
 
 namespace mgpu {
+extern unsigned g_spin_limit;      // krylov.cu: the spin_limit tuning key
+extern unsigned g_exchange_limit;  // krylov.cu: the exchange_spin_limit tuning key
 namespace {
 
 constexpr int kSweepThreads = 512;
@@ -69,6 +71,7 @@ struct Sweep {
     int nlev;        // local levels (those with a row of this block)
   } lo, up;
   int warps;         // warps that the widest of them needs
+  WaitLimits waits;
 };
 constexpr unsigned kPublish = 0x8000u;
 
@@ -303,11 +306,11 @@ __device__ __forceinline__ bool sweep_row(const Sweep<W>& S, const Fetched<W>& r
 #pragma unroll
   for (int t = 0; t < W; ++t) wait = wait || pending(v[t]);
   if (wait) {
-    unsigned spins = 0;
+    unsigned polls = S.waits.shared;
 #pragma unroll
     for (int t = 0; t < W; ++t)
       while (pending(v[t]) && ok) {
-        ok = keep_polling(spins, st);
+        ok = keep_polling(polls, st);
         v[t] = ld_value(r.c[t]);
       }
   }
@@ -354,7 +357,7 @@ __device__ __forceinline__ bool sweep_poll(const Sweep<W>& S, DevStatus* st) {
   unsigned left = 0u;
   for (int k = 0, j = tid; j < S.bw; j += P, ++k)
     if (first + j >= 0 && first + j < S.n) left |= 1u << k;
-  unsigned spins = 0;
+  unsigned polls = S.waits.value;
   while (left) {
     for (unsigned m = left; m; m &= m - 1u) {
       const int k = __ffs(m) - 1, j = tid + k * P;
@@ -365,7 +368,7 @@ __device__ __forceinline__ bool sweep_poll(const Sweep<W>& S, DevStatus* st) {
         left &= ~(1u << k);
       }
     }
-    if (left && !keep_polling(spins, st)) return false;
+    if (left && !keep_polling(polls, st)) return false;
   }
   return true;
 }
@@ -502,7 +505,9 @@ __device__ __forceinline__ bool grid_sum(Sweep<W>& S, VGrid& g, DevStatus* st, d
 }
 
 template <int W>
-__device__ __forceinline__ void sweep_begin(const KrylovArgs& a, const VGrid& g, Sweep<W>& S, int R, int vgrid) {
+__device__ __forceinline__ void sweep_begin(const KrylovArgs& a, const VGrid& g, Sweep<W>& S, int R, int vgrid,
+                                            WaitLimits waits) {
+  S.waits = waits;
   S.n = a.n;
   S.bw = a.bw;
   S.kind = a.precond;
@@ -522,11 +527,11 @@ __device__ __forceinline__ void sweep_begin(const KrylovArgs& a, const VGrid& g,
 
 // k_pcg (krylov.cu) with ILU(0) or IC(0)
 template <int W>
-__global__ void __launch_bounds__(kSweepThreads, 1) k_pcg_sweep(KrylovArgs a, int R, int vgrid) {
+__global__ void __launch_bounds__(kSweepThreads, 1) k_pcg_sweep(KrylovArgs a, int R, int vgrid, WaitLimits waits) {
   if (a.st->abort) return;
   VGrid g = whole_grid(a.bar, a.partials, true);
   Sweep<W> S;
-  sweep_begin<W>(a, g, S, R, vgrid);
+  sweep_begin<W>(a, g, S, R, vgrid, waits);
   double *x = a.x, *r = a.r, *p = a.p, *q = a.v, *z = a.r0;
   if (!sweep_prologue<W>(a, g, S)) return;
   double t[1];
@@ -605,11 +610,11 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_pcg_sweep(KrylovArgs a, in
 
 // k_bicgstab (krylov.cu) with ILU(0)
 template <int W>
-__global__ void __launch_bounds__(kSweepThreads, 1) k_bicgstab_sweep(KrylovArgs a, int R, int vgrid) {
+__global__ void __launch_bounds__(kSweepThreads, 1) k_bicgstab_sweep(KrylovArgs a, int R, int vgrid, WaitLimits waits) {
   if (a.st->abort) return;
   VGrid g = whole_grid(a.bar, a.partials, true);
   Sweep<W> S;
-  sweep_begin<W>(a, g, S, R, vgrid);
+  sweep_begin<W>(a, g, S, R, vgrid, waits);
   double *x = a.x, *r = a.r, *r0 = a.r0, *p = a.p, *v = a.v, *s = a.s, *t = a.t, *ph = a.ph, *sh = a.sh;
   if (!sweep_prologue<W>(a, g, S)) return;
   double t1[1];
@@ -748,7 +753,8 @@ int launch_sweep(const KrylovArgs& a, bool pcg, cudaStream_t s, bool* taken) {
   MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 2048));
   KrylovArgs aa = a;
   int block = 0, RR = R, vgrid = krylov_grid(a.n, block, pcg ? 0 : 1);
-  void* args[] = {&aa, &RR, &vgrid};
+  WaitLimits waits = wait_limits(g_spin_limit, g_exchange_limit);
+  void* args[] = {&aa, &RR, &vgrid, &waits};
   MGPU_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
   MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3((a.n + R - 1) / R), dim3(kSweepThreads), args, (size_t)dyn, s));
   *taken = true;
