@@ -135,6 +135,14 @@ __global__ void k_csr_pattern(int n, const int* __restrict__ rp1, const int* __r
   atomicMax(&flags[kFar], far);
 }
 
+// Every row's entries lie within the arrays (the device reads them unchecked).
+int check_rows(int n, const int32_t* row_ptr) {
+  bool ok = true;
+  for (int i = 0; i <= n; ++i) ok = ok && row_ptr[i] >= 1 && row_ptr[i] <= row_ptr[n];
+  if (!ok) set_error("CSR matrix: a row pointer out of range");
+  return ok ? 0 : MGPU_E_ARG;
+}
+
 int load_pattern(int n, const int32_t* row_ptr, const int32_t* col_idx, DevBuf& B, Pattern& P) {
   P.nnz = row_ptr[n] - 1;
   int *rp1, *col1, *flags;
@@ -300,6 +308,7 @@ int mgpu_krylov_solve(int n, const int32_t* row_ptr, const int32_t* col_idx, con
     set_error("mgpu_krylov_solve: invalid argument");
     return MGPU_E_ARG;
   }
+  TRY(check_rows(n, row_ptr));
   DevBuf B;
   const size_t nz = row_ptr[n] - 1;
   TRY(B.reserve(40 * nz + 220 * (size_t)n + (1 << 18)));
@@ -423,6 +432,7 @@ int mgpu_pcg_poly_solve(int n, const int32_t* row_ptr, const int32_t* col_idx, c
     set_error("mgpu_pcg_poly_solve: invalid argument");
     return MGPU_E_ARG;
   }
+  TRY(check_rows(n, row_ptr));
   DevBuf B;
   const size_t nz = row_ptr[n] - 1;
   TRY(B.reserve(32 * nz + 520 * (size_t)n + (1 << 18)));
