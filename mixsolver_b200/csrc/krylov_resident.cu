@@ -1211,7 +1211,8 @@ int fit_rows(int n, int W, int ld, const int* ell_col, int bw, int R, int room, 
   const int WC = W <= 5 ? 5 : 7, flags = 4 * resident_window_words(R, bw);
   const int T = block_threads(R), K = thread_rows(R);
   fits = false;
-  if (resident_smem(WC, R, bw, 0, K * (T / 32)) > room || flags > 48 * 1024) return 0;
+  if (resident_smem(WC, R, bw, 0, K * (T / 32)) > room) return 0;
+  if (flags + (int)sizeof(int) > 48 * 1024) return 0;  // with the kernel's own sum, a block's shared memory unasked
   MGPU_CUDA(cudaMemsetAsync(most, 0, sizeof(int), s));
   k_halo_words<<<(n + R - 1) / R, 256, flags, s>>>(n, W, ld, ell_col, bw, R, most);
   MGPU_CUDA(cudaGetLastError());

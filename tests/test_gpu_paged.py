@@ -86,3 +86,15 @@ def test_paged_solves_bit_exact(name):
         np.testing.assert_array_equal(x, y, err_msg=str((tol, maxit, degree)))
     x, it, res, ierr = S.pcg_poly(*paired, np.zeros_like(b), x0, 1e-9, 10)
     assert (it, res, ierr) == (0, 0.0, 0) and not x.any()
+
+
+def test_window_beyond_the_flags_is_streamed():
+    """A reach of 196,200 rows makes 12,288 window words, 48 KB of flags in the
+    kernel that counts the halo: not divided, and solved all the same."""
+    n, reach = 196_400, 196_200
+    lo = np.concatenate([np.arange(n - 1), [0]])
+    hi = np.concatenate([np.arange(1, n), [reach]])
+    paired, unpaired, b = _system(n, lo, hi)
+    got, want = (S.pcg_poly(*m, b, np.zeros(n), 1e-9, 400) for m in (paired, unpaired))
+    assert got[1:] == want[1:] and got[3] == 0
+    np.testing.assert_array_equal(got[0], want[0])
