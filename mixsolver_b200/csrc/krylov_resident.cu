@@ -675,11 +675,11 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // and a block's turn at page p + nb starts after its last step at p, of rank
 // p + steps r < p + nb + r while (steps - 1) r < nb (the plan keeps to half of
 // that); a sweep never waits for a later one. The other vectors stream.
-// Measured on a B200, a solve streamed -> here: 2,000,376 rows of 7 entries, 35
-// iterations at degree 48, 54.2 -> 46.4 ms; 3,072,000 rows of 5, 53 iterations,
-// 100.3 -> 96.4 ms. A step of a page takes 1.7 us of shared-memory reads and 2.9 us
-// of exchange (1.9 in the resident solve: here L2 also carries the pages), a turn
-// 4.8 us to load.
+// Measured on a B200, an iteration at degree 48 streamed -> here: 2,000,376 rows of
+// 7 entries 1,541 -> 1,234 to 1,315 us, 2,500,000 rows of 5 (a grid) 1,569 -> 974 to
+// 1,074 us (more sizes at turns_pay). A step of a page takes 1.7 us of shared-memory reads and 2.9 us of
+// exchange (1.9 in the resident solve: here L2 also carries the pages), a turn 4.8 us
+// to load.
 template <int WC, int K>
 __global__ void __launch_bounds__(256, 2) k_pcg_paged(KrylovArgs a, MixedArgs m, WaitLimits waits) {
   if (a.st->abort) return;
@@ -1221,6 +1221,33 @@ int fit_rows(int n, int W, int ld, const int* ell_col, int bw, int R, int room, 
   fits = resident_smem(WC, R, bw, words, K * (T / 32)) <= room && 4 * (R + 32 * words) <= 65535;
   return 0;
 }
+
+// Bytes of a streamed polynomial step: ELL columns and values, the vectors of a pass.
+double pass_bytes(int n, int W) { return (double)n * (8.0 * W + 56.0); }
+
+// Below this many bytes a step the streamed solve still hits L2 and is the faster
+// one whatever the pages' reach (hexahedra of 141 MB: 0.94 to 1.05 times as fast in
+// turns, of 162 MB 1.06 to 1.17).
+constexpr double kTurnBytes = 150e6;
+
+// Whether a larger system is solved faster in turns than streamed; steps: page
+// steps a block spends on a polynomial step of one page, loads and waits included.
+// Both times of a polynomial step follow 65 systems timed both ways on several
+// B200s. The streamed pass hardly differs between them; a page step, most of it
+// exchange through L2, takes 3.6 to 5.0 us with 7 entries a row, 4.2 to 5.4 with 5. us
+// an iteration, streamed / in turns, the fastest and the slowest seen: hexahedra in
+// natural order, 1.44M rows 1,033 / 921, 975, 2.0M 1,541 / 1,234, 1,315, 4.1M 2,906 / 2,478,
+// 2,643; in RCM order 2.0M 1,546 / 1,188, 1,276; mixed within 500 rows 1,650 / 1,790
+// (refused); a 1000 x 2500 grid 1,569 / 974, 1,074; tetrahedra in natural order, 1.7M 1,030 /
+// 1,049, 3.4M 2,034 / 2,289 (refused). Tetrahedra in RCM order lie on the line, 1.7M 1,022 /
+// 983, 1,090, 3.07M 1,841 / 1,781, 2,060; a PISO step on the 3.07M took 220.8 / 211.1 ms,
+// 216.9 / 213.8 on another GPU, its pressure solves 197.1 / 202.3 on a third.
+bool turns_pay(int n, int W, int R, int blocks, double steps) {
+  const bool wide = W > 5;
+  const double streamed = pass_bytes(n, W) / (wide ? 7.3e6 : 7.6e6);  // us
+  const double turns = std::ceil((double)n / R) / blocks + 0.5;  // the last turn has fewer pages than blocks
+  return turns * steps * (wide ? 4.3 : 4.55) <= streamed;
+}
 }  // namespace
 
 // The division of a system over the SMs for its resident solves: rows of a
@@ -1258,13 +1285,11 @@ int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan
     if (fits) keep(single * kSuperRows);
     if (fits) return 0;
   }
+  if (g_resident_sms == 0 && pass_bytes(n, W) < kTurnBytes) return 0;
   // pages: the largest that fits in half an SM, and the steps that make the most
   // of the shared memory. With G blocks, r pages of reach and a load that takes as
-  // long as L steps, steps pass at s (G - (s - 1) r) / (L + s) pages a step time
-  // (each page waits (s - 1) r pages' worth for those ahead of it). L = 2 fits a
-  // B200 (3,072,000 rows, r = 5.2: 111, 102, 96, 94 ms at 3, 5, 8, 10 steps); the
-  // streamed pass took about 2.3 G page-step times, so the turns are used while
-  // they promise a fifth less than that.
+  // long as L = 2 steps, steps pass at s (G - (s - 1) r) / (L + s) pages a step time
+  // (each page waits (s - 1) r pages' worth for those ahead of it).
   const int most = 2 * sms;
   for (int sc = kPageMax; sc >= kPageMin && !fits; --sc) {
     const int R = sc * kSuperRows;
@@ -1280,7 +1305,7 @@ int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan
         plan.steps = st;
       }
     }
-    if (best <= 0.0 || (g_resident_sms == 0 && most / best > 0.8 * 2.3)) {
+    if (best <= 0.0 || (g_resident_sms == 0 && !turns_pay(n, W, R, most, most / best))) {
       plan = ResidentPlan{};
       return 0;
     }

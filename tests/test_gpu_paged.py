@@ -8,6 +8,8 @@ on. The same system goes to the streaming kernel with one more entry, of value
 zero and without a transposed one: only symmetric patterns are divided."""
 import numpy as np
 import pytest
+import torch
+from torch.profiler import ProfilerActivity, profile
 
 from mixsolver_b200 import solver as S
 
@@ -98,3 +100,18 @@ def test_window_beyond_the_flags_is_streamed():
     got, want = (S.pcg_poly(*m, b, np.zeros(n), 1e-9, 400) for m in (paired, unpaired))
     assert got[1:] == want[1:] and got[3] == 0
     np.testing.assert_array_equal(got[0], want[0])
+
+
+# 524,288 rows mixed within 500: does not fit in shared memory, still hits L2 (in turns an
+# iteration took 380 us instead of 214); 1.44M rows: beyond L2 (921 us instead of 1,033)
+@pytest.mark.parametrize("box, window, kernel", [((128, 64, 64), 500, "k_pcg_mixed"),
+                                                 ((113, 113, 113), 0, "k_pcg_paged")])
+def test_turns_only_where_they_pay(box, window, kernel):
+    S.set_tuning("resident_sms", 0)
+    paired, _, b = _system(*_graph(*box, window))
+    torch.zeros(1).cuda()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        S.pcg_poly(*paired, b, np.zeros_like(b), 1e-8, 3)
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "k_pcg" in e.name]
+    assert names and all(kernel in k for k in names), names
