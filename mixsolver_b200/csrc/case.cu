@@ -25,6 +25,8 @@
 
 namespace mgpu {
 size_t page_floats(int n, int W, const ResidentPlan& plan);  // krylov_resident.cu
+int plan_sweep(int n, int width, int bw, int nlo, const int* lo_ptr, const int* lo_rows, int nup, const int* up_ptr,
+               const int* up_rows, int* scratch, cudaStream_t s, bool& pays);  // krylov_sweep.cu
 
 static thread_local std::string g_err;
 static int g_device = 0;
@@ -815,8 +817,12 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
   // allocation maps it again)
   if (!poly) {
     int wide = 0;
-    if ((e = device_row_extent(d.N, d.row_ptr, d.col, wide, d.bw, d.width, (int*)d.partials, c->stream)))
+    bool sweeps = false;
+    if ((e = device_row_extent(d.N, d.row_ptr, d.col, wide, d.bw, d.width, (int*)d.partials, c->stream)) ||
+        (e = plan_sweep(d.N, d.width, d.bw, d.nlev_lo, d.lo_ptr, d.lo_rows, d.nlev_up, d.up_ptr, d.up_rows,
+                        (int*)d.partials, c->stream, sweeps)))
       return fail(e);
+    if (!sweeps) d.width = 0;
   }
   if (ctrl->precision == MGPU_PREC_MIXED) {
     if ((e = plan_resident(d.N, d.ell_w, d.ell_ld, d.ell_col, far, d.plan, d.ferr, c->stream))) return fail(e);

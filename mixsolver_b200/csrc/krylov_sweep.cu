@@ -726,37 +726,118 @@ const void* sweep_kernel(bool pcg) {
   return pcg ? (const void*)k_pcg_sweep<W> : (const void*)k_bicgstab_sweep<W>;
 }
 
-// The resident solve of a factored system whose rows have at most 6 entries on
-// either side of the diagonal and fit in the SMs' shared memory, with the 6 n
-// more work doubles that a.width > 0 stands for; *taken = false and no launch
-// otherwise. As few blocks as hold the rows. It was the faster one at every size
-// measured, 4,096 to 65,536 rows (2.3 to 6 times a solve), so a system that fits
-// always takes it.
-int launch_sweep(const KrylovArgs& a, bool pcg, cudaStream_t s, bool* taken) {
-  *taken = false;
-  if (a.precond == 1 || a.width < 1 || a.width > 6) return 0;
-  int dev = 0, sms = 0, smem = 0;
+namespace {
+
+// The division of a system whose rows have at most 6 entries on either side of
+// the diagonal: rows of a block, as few blocks as hold them. False when the rows
+// do not fit in the SMs' shared memory.
+struct SweepDivision {
+  int W, R, blocks, smem;
+};
+int divide_sweep(int n, int width, int bw, SweepDivision& v, bool& fits) {
+  fits = false;
+  if (width < 1 || width > 6) return 0;
+  int dev = 0, sms = 0;
   MGPU_CUDA(cudaGetDevice(&dev));
   MGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  MGPU_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const int W = a.width <= 3 ? 3 : a.width == 4 ? 4 : 6;
-  const long room = smem - 2048 - sweep_smem(W, 0, a.bw);
-  const int most = room > 0 ? (int)(room / sweep_row_bytes(W) / 32 * 32) : 0;
+  MGPU_CUDA(cudaDeviceGetAttribute(&v.smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  v.W = width <= 3 ? 3 : width == 4 ? 4 : 6;
+  const long room = v.smem - 2048 - sweep_smem(v.W, 0, bw);
+  const int most = room > 0 ? (int)(room / sweep_row_bytes(v.W) / 32 * 32) : 0;
   // the polling threads keep their rows in a 32-bit mask; places are 16 bits
-  if (most < 256 || a.bw > 32 * 32 * kPollWarps) return 0;
-  const int blocks = (a.n + most - 1) / most;
-  const int R = ((a.n + blocks - 1) / blocks + 31) / 32 * 32;
-  if (blocks > sms) return 0;
-  const int dyn = (int)sweep_smem(W, R, a.bw);
-  const void* fn = W == 3 ? sweep_kernel<3>(pcg) : W == 4 ? sweep_kernel<4>(pcg) : sweep_kernel<6>(pcg);
+  if (most < 256 || bw > 32 * 32 * kPollWarps) return 0;
+  const int blocks = (n + most - 1) / most;
+  v.R = ((n + blocks - 1) / blocks + 31) / 32 * 32;
+  v.blocks = (n + v.R - 1) / v.R;
+  fits = blocks <= sms;
+  return 0;
+}
+
+// The most rows that a level (rows ascending) has in one block: a thread a level and block.
+__global__ void k_widest_level(int nlo, const int* __restrict__ lo_ptr, const int* __restrict__ lo_rows, int nup,
+                               const int* __restrict__ up_ptr, const int* __restrict__ up_rows, int R, int blocks,
+                               int* widest) {
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  int mine = 0;
+  if (t < (long)(nlo + nup) * blocks) {
+    const int lev = (int)(t / blocks), blk = (int)(t % blocks);
+    const int* ptr = lev < nlo ? lo_ptr + lev : up_ptr + (lev - nlo);
+    const int* rows = lev < nlo ? lo_rows : up_rows;
+    auto below = [&](long key) {
+      int lo = ptr[0], hi = ptr[1];
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (rows[mid] < key)
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      return lo;
+    };
+    mine = below((blk + 1l) * R) - below((long)blk * R);
+  }
+  mine = __reduce_max_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0 && mine > 0) atomicMax(widest, mine);
+}
+
+}  // namespace
+
+// Whether a system's sweeps are faster here than in krylov.cu (the caller then
+// passes its width on in KrylovArgs, 0 otherwise). Each of the blocks polls bw
+// values with the threads that no level needs, one after another, and a value
+// waits half a round of them: blocks * bw / pollers against the levels, whose
+// cost in krylov.cu is a grid-wide hop each. Measured on a B200 as krylov.cu's
+// time over this one's, a BiCGStab+ILU(0) iteration (PCG+IC(0) gains more), by
+// that quotient: channels of n = 65k, 100k, 126k, 151k, 180k, 216k rows in RCM
+// order, at 1.8, 3.6, 5.3, 7.1, 9.3, 12: 2.5, 1.8, 1.4, 1.1, 0.98, 0.87; tetrahedra
+// in natural order, 5.4 and 11: 1.4 and 0.98. Up to 8 it pays. Tetrahedra in RCM
+// order, whose levels cross most blocks: 1.2 with 98 blocks (2.8), 0.97 with 129
+// (4.0); narrow levels keep paying there: hexahedra in natural order, 130 blocks,
+// at most 36 rows of a level in a block (5.4): 3.6. scratch: one int on the device;
+// waits for stream s only where the answer depends on the widest level.
+int plan_sweep(int n, int width, int bw, int nlo, const int* lo_ptr, const int* lo_rows, int nup, const int* up_ptr,
+               const int* up_rows, int* scratch, cudaStream_t s, bool& pays) {
+  constexpr long kRounds = 8;
+  constexpr int kManyBlocks = 120, kNarrow = 64;
+  SweepDivision v;
+  if (int e = divide_sweep(n, width, bw, v, pays)) return e;
+  if (!pays) return 0;
+  const long polls = (long)v.blocks * bw, levels = std::min(nlo, nup);
+  const int fewest = 32 * kPollWarps;
+  if (v.blocks <= kManyBlocks && polls <= kRounds * fewest * levels) return 0;
+  int widest = 0;
+  const long threads = (long)(nlo + nup) * v.blocks;
+  MGPU_CUDA(cudaMemsetAsync(scratch, 0, sizeof(int), s));
+  k_widest_level<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(nlo, lo_ptr, lo_rows, nup, up_ptr, up_rows, v.R,
+                                                                  v.blocks, scratch);
+  MGPU_CUDA(cudaGetLastError());
+  MGPU_CUDA(cudaMemcpyAsync(&widest, scratch, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MGPU_CUDA(cudaStreamSynchronize(s));
+  const int pollers = std::max(kSweepThreads - (widest + 31) / 32 * 32, fewest);
+  pays = polls <= kRounds * pollers * levels && (v.blocks <= kManyBlocks || widest <= kNarrow);
+  return 0;
+}
+
+// The resident solve of a factored system that plan_sweep has found worth it,
+// with the 6 n more work doubles that a.width > 0 stands for; *taken = false and
+// no launch otherwise.
+int launch_sweep(const KrylovArgs& a, bool pcg, cudaStream_t s, bool* taken) {
+  *taken = false;
+  SweepDivision v;
+  bool fits = false;
+  if (a.precond == 1) return 0;
+  if (int e = divide_sweep(a.n, a.width, a.bw, v, fits)) return e;
+  if (!fits) return 0;
+  const int dyn = (int)sweep_smem(v.W, v.R, a.bw);
+  const void* fn = v.W == 3 ? sweep_kernel<3>(pcg) : v.W == 4 ? sweep_kernel<4>(pcg) : sweep_kernel<6>(pcg);
   // the same limit on every call: another thread may be launching the kernel for another system
-  MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 2048));
+  MGPU_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem - 2048));
   KrylovArgs aa = a;
-  int block = 0, RR = R, vgrid = krylov_grid(a.n, block, pcg ? 0 : 1);
+  int block = 0, RR = v.R, vgrid = krylov_grid(a.n, block, pcg ? 0 : 1);
   WaitLimits waits = wait_limits(g_spin_limit, g_exchange_limit);
   void* args[] = {&aa, &RR, &vgrid, &waits};
   MGPU_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), s));
-  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3((a.n + R - 1) / R), dim3(kSweepThreads), args, (size_t)dyn, s));
+  MGPU_CUDA(cudaLaunchCooperativeKernel(fn, dim3(v.blocks), dim3(kSweepThreads), args, (size_t)dyn, s));
   *taken = true;
   return 0;
 }

@@ -21,6 +21,8 @@ extern double g_cheb_ratio;
 void cheb_params(long n, int& k, double& ratio);  // krylov.cu
 extern int g_prefetch_mb;      // l2_prefetch_mb
 size_t page_floats(int n, int W, const ResidentPlan& plan);  // krylov_resident.cu
+int plan_sweep(int n, int width, int bw, int nlo, const int* lo_ptr, const int* lo_rows, int nup, const int* up_ptr,
+               const int* up_rows, int* scratch, cudaStream_t s, bool& pays);  // krylov_sweep.cu
 }
 
 using namespace mgpu;
@@ -392,7 +394,10 @@ int mgpu_krylov_solve(int n, const int32_t* row_ptr, const int32_t* col_idx, con
   a.tol = tol;
   a.maxit = maxit;
   a.precond = precond;
-  a.width = P.width;
+  bool sweeps = false;
+  if (precond != 1)
+    TRY(plan_sweep(n, P.width, P.bw, L.nlo, dlop, dlor, L.nup, dupp, dupr, dferr, 0, sweeps));
+  a.width = sweeps ? P.width : 0;
   a.bw = P.bw;
   a.zero_x = 0;
   a.mpi_mode = norm_mode ? 1 : 0;
