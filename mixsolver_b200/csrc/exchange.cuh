@@ -52,7 +52,7 @@ constexpr unsigned kSharedSpins = 1u << 26;
 struct WaitLimits {
   unsigned barrier, value, shared;
 };
-inline WaitLimits wait_limits(unsigned spin_limit, unsigned exchange_limit) {
+__host__ __device__ constexpr WaitLimits wait_limits(unsigned spin_limit, unsigned exchange_limit) {
   return {spin_limit ? spin_limit : kHaloSpins, exchange_limit ? exchange_limit : kHaloSpins,
           exchange_limit ? exchange_limit : kSharedSpins};
 }
