@@ -25,6 +25,7 @@
 
 namespace mgpu {
 size_t page_floats(int n, int W, const ResidentPlan& plan);  // krylov_resident.cu
+bool may_take_pages(int n, int W);
 int plan_sweep(int n, int width, int bw, int nlo, const int* lo_ptr, const int* lo_rows, int nup, const int* up_ptr,
                const int* up_rows, int* scratch, cudaStream_t s, bool& pays);  // krylov_sweep.cu
 
@@ -709,6 +710,7 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
       d.ell_w = w;
       d.ell_ld = (int)ld;
     }
+    if (ctrl->precision == MGPU_PREC_MIXED && !may_take_pages(d.N, w) && (e = c->alloc(d.a32, d.nnz))) return fail(e);
   }
   // geometry (device), scratch for the node arrays and provisional centres
   std::vector<int> fptr_h(hm.fptr.begin(), hm.fptr.end());
@@ -826,8 +828,10 @@ int mgpu_case_create(const MgpuMesh* mesh, const MgpuCtrl* ctrl, MgpuCase** out,
   }
   if (ctrl->precision == MGPU_PREC_MIXED) {
     if ((e = plan_resident(d.N, d.ell_w, d.ell_ld, d.ell_col, far, d.plan, d.ferr, c->stream))) return fail(e);
-    // the pages of a larger system's pressure solve follow its CSR values
-    if ((e = c->alloc(d.a32, d.nnz + page_floats(d.N, d.ell_w, d.plan)))) return fail(e);
+    // the pages of a larger system's pressure solve follow its CSR values; the others have theirs (an
+    // allocation this late took 2 ms of the 76 that a 729k-cell case takes to create)
+    if (d.a32 && d.plan.steps > 0) d.plan = ResidentPlan{};  // resident_sms was set meanwhile: no room for pages
+    if (!d.a32 && (e = c->alloc(d.a32, d.nnz + page_floats(d.N, d.ell_w, d.plan)))) return fail(e);
   }
   // scalars needing a sequential pass: flux_ref (group/face order) and the
   // smallest vol**(1/3) (CFL estimate); computed once on the host

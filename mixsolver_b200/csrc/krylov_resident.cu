@@ -1250,6 +1250,9 @@ bool turns_pay(int n, int W, int R, int blocks, double steps) {
 }
 }  // namespace
 
+// Whether plan_resident may give pages to a system, by its size alone.
+bool may_take_pages(int n, int W) { return W <= 7 && (g_resident_sms > 0 || pass_bytes(n, W) >= kTurnBytes); }
+
 // The division of a system over the SMs for its resident solves: rows of a
 // block (whole super-chunks) and the most halo words of a block; larger systems:
 // the largest page and the steps of its turn. No plan (rows 0) with more than 7
@@ -1285,7 +1288,7 @@ int plan_resident(int n, int W, int ld, const int* ell_col, int bw, ResidentPlan
     if (fits) keep(single * kSuperRows);
     if (fits) return 0;
   }
-  if (g_resident_sms == 0 && pass_bytes(n, W) < kTurnBytes) return 0;
+  if (!may_take_pages(n, W)) return 0;
   // pages: the largest that fits in half an SM, and the steps that make the most
   // of the shared memory. With G blocks, r pages of reach and a load that takes as
   // long as L = 2 steps, steps pass at s (G - (s - 1) r) / (L + s) pages a step time
