@@ -139,10 +139,11 @@ __global__ void k_csr_pattern(int n, const int* __restrict__ rp1, const int* __r
 
 // Every row's entries lie within the arrays (the device reads them unchecked).
 int check_rows(int n, const int32_t* row_ptr) {
-  bool ok = true;
-  for (int i = 0; i <= n; ++i) ok = ok && row_ptr[i] >= 1 && row_ptr[i] <= row_ptr[n];
-  if (!ok) set_error("CSR matrix: a row pointer out of range");
-  return ok ? 0 : MGPU_E_ARG;
+  const int end = row_ptr[n];
+  int bad = end < 1;
+  for (int i = 0; i <= n; ++i) bad |= (row_ptr[i] < 1) | (row_ptr[i] > end);  // no early exit: it vectorises
+  if (bad) set_error("CSR matrix: a row pointer out of range");
+  return bad ? MGPU_E_ARG : 0;
 }
 
 int load_pattern(int n, const int32_t* row_ptr, const int32_t* col_idx, DevBuf& B, Pattern& P) {
