@@ -464,15 +464,18 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": None,
-                     "resident": "shared memory: the FP32 matrix stays in the SMs' shared memory for the whole "
-                                 "solve and only the values that blocks exchange travel through L2; the "
-                                 "algorithmic bytes count it once a pass, so frac is an HBM-equivalent rate and "
-                                 "may exceed 1; see l2 for the fraction of the L2 roofline",
+                     "resident": "a system that fits (up to about 570,000 rows of 7 entries) keeps its FP32 matrix "
+                                 "in the SMs' shared memory for the whole solve and is bound by shared-memory "
+                                 "reads and the exchange between blocks; the algorithmic bytes count the matrix "
+                                 "once a pass, so frac is an HBM-equivalent rate and may exceed 1; see l2 for the "
+                                 "fraction of the L2 roofline" if mixed else None,
                      "l2": {"achieved": achieved, "peak": l2peak, "unit": "GB/s",
                             "frac": (achieved / l2peak) if achieved else None,
                             "peak_source": "L2-resident c = a + b over 3 x 16 MiB buffers, graph-replayed, "
                                            "measured in this run"},
-                     "kernel": "k_pcg_resident (pressure solve)" if mixed else "k_factor+k_pcg (pressure solve)",
+                     "kernel": "pressure solve: k_pcg_resident where the system fits in shared memory, else k_pcg_paged "
+                               "or k_pcg_mixed" if mixed else
+                               "pressure solve: k_factor, then k_pcg_sweep where it pays, else k_pcg",
                      "algorithmic_bytes_per_launch": float(np.mean(ppe_bytes)), "avg_launch_ms": ppe_launch_ms,
                      "launches": len(ppe_ms), "all_krylov_solves_gbs": family,
                      "peak_source": peak_source},
@@ -660,7 +663,8 @@ def run_piso(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": None,
-                     "kernel": "k_pcg_paged (pressure solves; k_pcg_resident up to about 820,000 tets)",
+                     "kernel": "pressure solves: k_pcg_resident where the system fits in shared memory (up to about "
+                               "680,000 tets), else k_pcg_paged where turns pay, else k_pcg_mixed",
                      "algorithmic_bytes_per_launch": float(np.mean(ppe_bytes)), "avg_launch_ms": ppe_launch_ms,
                      "launches": len(ppe_ms), "all_krylov_solves_gbs": family,
                      "peak_source": peak_source},
