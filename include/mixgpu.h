@@ -359,7 +359,9 @@ int mgpu_cg_jacobi_noalloc(int n, const int32_t* d_row_ptr, const int32_t* d_col
  * systems that fit in the SMs' shared memory are divided by their size alone),
  * "sweep_threads" (threads of a sync-free triangular sweep, default 65536),
  * "sweep_sleep_ns" (back-off of a long wait in that sweep, default 0),
- * "min_blocks" (least number of blocks of a multi-block solve, default 1),
+ * "min_blocks" (least number of blocks of a multi-block solve, default 1; FP64
+ * factored systems solved in the SMs' shared memory take no part in the sweep_*
+ * keys, and single_block_rows and min_blocks only choose the order of their sums),
  * "cheb_degree" (mixed form: degree of the Chebyshev-Jacobi pressure
  * preconditioner, 1 = plain Jacobi, default 24), "cheb_ratio" (lambda_max over
  * lambda_min of its interval, default 1000), "cheb_large_rows",
